@@ -188,7 +188,7 @@ int alloc_particles(mf_ctx *ctx, int N) {
   TRY(alloc_set(ctx, ctx->set[1], N));
   dev_buffers &D = ctx->D;
   TRY(dalloc(ctx, L, &D.n, N));
-  TRY(dalloc(ctx, L, &D.rec, (size_t)N * R_WIDTH));
+  TRY(dalloc(ctx, L, &D.rec, rec_doubles(N) + (size_t)N * 2));  // pair records, candidate records
   TRY(dalloc(ctx, L, &D.recf, (size_t)N * F_WIDTH));
   TRY(dalloc(ctx, L, &D.S_der, N));
   TRY(dalloc(ctx, L, &D.v_der, N));
@@ -264,6 +264,9 @@ void set_list_mode(mf_ctx *ctx) {
   // the EOS sound speed of every particle: the device's float rounding of the same IEEE
   // operations, computed once
   ctx->P.eos_c0 = (double)sqrtf((float)(ctx->P.phys.K / ctx->P.phys.rho0));
+  ctx->P.inv_wdeltap = 1. / ctx->P.corr.wdeltap;
+  ctx->P.alpha_half = 0.5 * ctx->P.corr.alpha;
+  ctx->P.eta2 = ctx->P.corr.eta * ctx->P.corr.eta;
   ctx->P.verlet = list_mode(ctx) ? 1 : 0;
   ctx->P.fuse = ctx->P.verlet && (ctx->flags & MF_OPT_FUSED_PREDICTOR) ? 1 : 0;
   // at most half a cell: the lists are built over the 7x7 cells around a particle, which hold
@@ -322,6 +325,15 @@ int launch_cells(mf_ctx *ctx, bool step_mode) {
   return MF_OK;
 }
 
+int launch_pair_fp64(mf_ctx *ctx) {
+  const int lanes = pair64_lanes(ctx->N), per = PAIR64_BLOCK / lanes, nb = (ctx->N + per - 1) / per;
+  switch (lanes) {
+    case 4: return launch_pdl(ctx, k_pair_fp64<4>, nb, PAIR64_BLOCK, ctx->P, ctx->D);
+    case 2: return launch_pdl(ctx, k_pair_fp64<2>, nb, PAIR64_BLOCK, ctx->P, ctx->D);
+    default: return launch_pdl(ctx, k_pair_fp64<1>, nb, PAIR64_BLOCK, ctx->P, ctx->D);
+  }
+}
+
 int launch_stage(mf_ctx *ctx, int stage) {
   static const char *const names[4] = {"mf stage 0: cell list", "mf stage 1: predictor",
                                        "mf stage 2: pair sums", "mf stage 3: finish + return map"};
@@ -343,7 +355,7 @@ int launch_stage(mf_ctx *ctx, int stage) {
     case 2:
       if (mixed && ctx->P.verlet) TRY(launch_pdl(ctx, k_pair_mixed<true>, npb, PAIR_BLOCK, ctx->P, ctx->D));
       else if (mixed) TRY(launch_pdl(ctx, k_pair_mixed<false>, npb, PAIR_BLOCK, ctx->P, ctx->D));
-      else TRY(launch_pdl(ctx, k_pair_fp64, (N + PAIR64_BLOCK - 1) / PAIR64_BLOCK, PAIR64_BLOCK, ctx->P, ctx->D));
+      else TRY(launch_pair_fp64(ctx));
       if (ctx->P.thermal_solver == MF_THERMAL_PSE && ctx->P.thermal_wp) {
         if (mixed) TRY(launch_pdl(ctx, k_pse_mixed, npb, PAIR_BLOCK, ctx->P, ctx->D));
         else TRY(launch_pdl(ctx, k_pse, npb, PAIR_BLOCK, ctx->P, ctx->D));
@@ -700,10 +712,10 @@ int mf_get_field(mf_ctx *ctx, int field, void *host) {
       }
       return MF_OK;
     }
-    std::vector<double> rec(N * R_WIDTH);
-    CK(cudaMemcpy(rec.data(), ctx->D.rec, sizeof(double) * N * R_WIDTH, cudaMemcpyDeviceToHost));
+    std::vector<double> rec(rec_doubles((int)N));
+    CK(cudaMemcpy(rec.data(), ctx->D.rec, sizeof(double) * rec.size(), cudaMemcpyDeviceToHost));
     for (size_t i = 0; i < N; ++i) {
-      auto at = [&](int f) { return rec[(size_t)(f / 2) * N * 2 + (size_t)i * 2 + f % 2]; };
+      auto at = [&](int f) { return rec[2 * rec_word(f / 2, (int)i) + f % 2]; };
       o[4 * i] = at(R_RXX);
       o[4 * i + 1] = at(R_RXY);
       o[4 * i + 2] = at(R_RYY);
@@ -1143,7 +1155,9 @@ int batch_build_fused(mf_batch *b, int K) {
     c->cur = saved;
     bind_sets(c);
     const int pair_bs = b->form == MF_BATCH_PERSISTENT ? PERSIST_BLOCK : b->pair_bs;
-    const int blocks[4] = {c->scan_tiles, (c->N + BLOCK - 1) / BLOCK, (c->N + pair_bs - 1) / pair_bs,
+    // particles per pair block
+    const int per = pair_bs / (c->P.precision == MF_PRECISION_MIXED ? 1 : pair64_lanes(c->N));
+    const int blocks[4] = {c->scan_tiles, (c->N + BLOCK - 1) / BLOCK, (c->N + per - 1) / per,
                            (int)std::max<long long>(1, (long long)sms * PLASTIC_BLOCKS_PER_SM * c->N / total_n)};
     for (int m = 0; m < 4; ++m) first[(size_t)m * (n + 1) + k + 1] = first[(size_t)m * (n + 1) + k] + blocks[m];
   }

@@ -91,7 +91,12 @@ static __global__ void __launch_bounds__(BS) kb_pair_fp64(batch_map M) {
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  pair_fp64_body(s.P, s.D, b);
+  __shared__ unsigned s_list[pair64_shared<BS>::WORDS];
+  switch (pair64_lanes(s.P.N)) {  // the system's own rule, so that its sums are its own context's
+    case 4: pair_fp64_body<BS, 4>(s.P, s.D, b, s_list); break;
+    case 2: pair_fp64_body<BS, 2>(s.P, s.D, b, s_list); break;
+    default: pair_fp64_body<BS, 1>(s.P, s.D, b, s_list); break;
+  }
 }
 
 template <int BS>

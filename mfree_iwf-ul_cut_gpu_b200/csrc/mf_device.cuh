@@ -57,6 +57,7 @@ struct params {
   int verlet;
   int fuse;  // neighbour lists: the finish kernel also runs the next step's predictor
   float skin;
+  double inv_wdeltap, alpha_half, eta2;  // 1 / corr.wdeltap, corr.alpha / 2, corr.eta^2
   double eos_c0;  // (double)sqrtf((float)(K / rho0)), the EOS sound speed (actions_gpu.cu:41-51)
   double dt;
   // tool-workpiece contact conductance (an extension without a reference counterpart, off at

@@ -367,6 +367,26 @@ __device__ __forceinline__ int stable_rank(const int4 *__restrict__ perm_u, cons
   return r;
 }
 
+// FP64 pair records: eight 16-byte planes per particle in tiles of 32 particles (plane k of the
+// tile's particles together, 512 bytes), so that a warp's loads of one plane for neighbouring
+// particles are coalesced and one address serves all eight (the planes are constant offsets).
+__host__ __device__ __forceinline__ size_t rec_word(int k, int j) {
+  return (size_t)(j >> 5) * (R_WIDTH / 2 * 32) + (size_t)(k * 32 + (j & 31));
+}
+__device__ __forceinline__ double2 rec_plane(const double *__restrict__ rec, int k, int j) {
+  return __ldg(reinterpret_cast<const double2 *>(rec) + rec_word(k, j));
+}
+// The FP32 candidate records behind them, what the pair kernel's distance test reads: position
+// relative to the origin of the particle's own cell, marks | cell column, cell row. Blanked
+// particles sit at infinity, which no test takes; particles that have to be taken whatever their
+// distance (a NaN or Inf in the record, a position the FP32 offset cannot hold, a density outside
+// float's range) at NaN, which every test takes.
+constexpr unsigned CAND_TOOL = 0x80000000u, CAND_ANY = 0x40000000u, CAND_COLUMN = 0x3fffffffu;
+__host__ __device__ __forceinline__ size_t rec_doubles(int N) { return (size_t)((N + 31) / 32) * 32 * R_WIDTH; }
+__device__ __forceinline__ const float4 *rec_cand(const double *rec, int N) {
+  return reinterpret_cast<const float4 *>(rec + rec_doubles(N));
+}
+
 // gather into the new order (grid_gpu_green.cu:22-116) and, if PREDICT, the predictor
 // (leap_frog.cu:30-66), EOS (actions_gpu.cu:41-51), artificial stress (:53-97) and the
 // neighbour records read by the pair kernel.
@@ -449,10 +469,19 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     if (!finite) rf |= FLAG_NONFINITE;
     r[R_FLAGS] = __longlong_as_double((long long)rf);
     // the FP64 record feeds the FP64 pair kernel and its PSE pass (kept when staged, for reads);
-    // eight planes of double2 (structure of arrays): plane k of particle q at [k * N + q]
     double2 *dst = reinterpret_cast<double2 *>(D.rec);
 #pragma unroll
-    for (int k = 0; k < R_WIDTH / 2; ++k) dst[(size_t)k * P.N + q] = make_double2(r[2 * k], r[2 * k + 1]);
+    for (int k = 0; k < R_WIDTH / 2; ++k) dst[rec_word(k, q)] = make_double2(r[2 * k], r[2 * k + 1]);
+    // the candidate record; more than four cells from the cell it is counted in (a particle
+    // clamped to the grid) an FP32 offset would lose the digits the test needs
+    const geom g = *D.g;
+    const int ci = hsh / g.ny, cj = hsh - ci * g.ny;
+    const double rx = pos.x - (g.bbmin_x + ci * g.dx), ry = pos.y - (g.bbmin_y + cj * g.dx);
+    const bool any = (rf & FLAG_NONFINITE) || !(fabs(rx) <= 4. * g.dx && fabs(ry) <= 4. * g.dx) ||
+                     !(fabs(rho) >= 1e-30 && fabs(rho) <= 1e30) || !(h >= 1e-15 && h <= 1e15);
+    const_cast<float4 *>(rec_cand(D.rec, P.N))[q] =
+        make_float4(blanked ? __int_as_float(0x7f800000) : any ? __int_as_float(0x7fffffff) : (float)rx, (float)ry,
+                    __uint_as_float((unsigned)ci | (tool ? CAND_TOOL : 0u) | (any ? CAND_ANY : 0u)), (float)cj);
     const float fv[12] = {(float)vel.x, (float)vel.y, (float)sxx, (float)sxy, (float)syy, (float)Rxx,
                           (float)Rxy, (float)Ryy, (float)h, (float)rho, (float)c, (float)vol};
 #pragma unroll
@@ -636,183 +665,306 @@ static __global__ void __launch_bounds__(BLOCK, REORDER_BLOCKS_PER_SM) k_reorder
 // visiting the columns in x order and each range in array order is the reference's
 // neighbour order (x-cell outer, y-cell inner, sorted order within a cell).
 
-// plane k of the FP64 record of particle j
-__device__ __forceinline__ double2 rec_plane(const double *__restrict__ rec, int N, int k, int j) {
-  return __ldg(reinterpret_cast<const double2 *>(rec) + (size_t)k * N + j);
+// 1 / x for x within float's range by one third-order Newton step from the FP32 reciprocal
+// approximation y of x: its relative error, with x's rounding to float below 2e-7, cubed is below
+// 1e-20, so the result is rounded like a division to within the last bit, in three multiply-adds.
+__device__ __forceinline__ double rcp64_from(double x, float xf) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(xf));
+  const double y0 = (double)y;
+  const double r = fma(-x, y0, 1.);
+  return fma(y0, fma(r, r, r), y0);
 }
+__device__ __forceinline__ double rcp64(double x) { return rcp64_from(x, (float)x); }
 
-__device__ __forceinline__ void load_rec(const double *__restrict__ rec, int N, int j, double *r) {
-#pragma unroll
-  for (int k = 0; k < R_WIDTH / 2; ++k) {
-    const double2 v = rec_plane(rec, N, k, j);
-    r[2 * k] = v.x;
-    r[2 * k + 1] = v.y;
+// the i particle's values of the FP64 pair sums
+struct pair64_i {
+  double x, y, vx, vy, sxx, sxy, syy, Rxx, Rxy, Ryy, h, rho, c, T;
+  double h1, fourh2, fac, dw_in, dw_out, thermal_alpha;
+  bool tool, thermal;
+};
+// The sums, without their constant factors (applied once at the end): stress without the mass,
+// viscosity without -2 mass, XSPH without 2 mass eps, Brookshaw without 2
+struct pair64_acc {
+  double v[4], s[4], vt[2], xt[2], T;
+};
+
+// Neighbour j (its record's planes r[0..7]) added to particle i's sums (interactions_gpu.cu:147-345,
+// kernels.cuh:30-70). The reference's expressions with the divisions taken out of the pair: the
+// spline's 1 / r cancels for q <= 1 and comes from rcp64 beyond, 1 / rho_ij and the viscosity's
+// denominator from rcp64 (by division where a value may lie outside float's range: careful),
+// w / wdeltap by a reciprocal per particle. Both branches of the spline are evaluated (a warp's
+// lanes nearly always hold both). Every multiply-add is written out, so that each kernel that
+// inlines this rounds alike.
+__device__ __forceinline__ void pair64_add(const params &P, const pair64_i &I, const double2 r[8], bool tool_j, bool careful,
+                                           pair64_acc &a) {
+  const double xij = I.x - r[0].x, yij = I.y - r[0].y;
+  const double rr2 = fma(xij, xij, __dmul_rn(yij, yij));
+  // outside the support the reference adds terms times W = 0, which only a NaN / Inf survives:
+  // there the outer branch at t = 0
+  const bool in_support = !(rr2 >= I.fourh2 || rr2 < 1e-8);
+  const float radf = sqrtf((float)rr2);
+  const double rad = (double)radf;
+  const double q = __dmul_rn(rad, I.h1);
+  const bool out = q > 1. || !in_support;
+  const double t = in_support ? __dsub_rn(2., q) : 0.;
+  const double t2 = __dmul_rn(t, t);
+  const double val_out = __dmul_rn(__dmul_rn(t2, t2), __dmul_rn(0.25, t2));
+  const double val_in = fma(__dmul_rn(__dmul_rn(-1.5, q), q), fma(-0.5, q, 1.), 1.);
+  // (in the support r >= 1e-4; the bound keeps coincident particles' 1 / r finite)
+  const float rb = fmaxf(radf, 1e-18f);
+  const double der_out = __dmul_rn(__dmul_rn(I.dw_out, t2), rcp64_from((double)rb, rb));
+  const double der_in = __dmul_rn(I.dw_in, fma(-0.75, q, 1.));
+  const double w = __dmul_rn(out ? val_out : val_in, I.fac);
+  const double dwr = out ? der_out : der_in;
+  const double wx = __dmul_rn(dwr, xij), wy = __dmul_rn(dwr, yij);
+  const double volj = r[6].y;
+  if (!I.tool && !tool_j) {
+    const double dvx = __dsub_rn(r[1].x, I.vx), dvy = __dsub_rn(r[1].y, I.vy);
+    const double ax = __dmul_rn(dvx, volj), ay = __dmul_rn(dvy, volj);
+    a.v[0] = fma(ax, wx, a.v[0]);
+    a.v[1] = fma(ax, wy, a.v[1]);
+    a.v[2] = fma(ay, wx, a.v[2]);
+    a.v[3] = fma(ay, wy, a.v[3]);
+    double fab = __dmul_rn(w, P.inv_wdeltap);
+    fab = __dmul_rn(fab, fab);
+    fab = __dmul_rn(fab, fab);
+    const double sxx = fma(fab, __dadd_rn(I.Rxx, r[3].y), __dadd_rn(I.sxx, r[2].x));
+    const double sxy = fma(fab, __dadd_rn(I.Rxy, r[4].x), __dadd_rn(I.sxy, r[2].y));
+    const double syy = fma(fab, __dadd_rn(I.Ryy, r[4].y), __dadd_rn(I.syy, r[3].x));
+    a.s[0] = fma(sxx, wx, a.s[0]);
+    a.s[1] = fma(sxy, wy, a.s[1]);
+    a.s[2] = fma(sxy, wx, a.s[2]);
+    a.s[3] = fma(syy, wy, a.s[3]);
+    const double nvr = fma(dvx, xij, __dmul_rn(dvy, yij));  // -v_ij . x_ij
+    const double rs = __dadd_rn(I.rho, r[5].y);
+    const double hij = __dmul_rn(0.5, __dadd_rn(I.h, r[5].x));
+    const double den = fma(__dmul_rn(P.eta2, hij), hij, rr2);
+    double irho = rcp64(rs), iden = rcp64(den);  // half of 1 / rho_ij; 1 / (r^2 + eta^2 h_ij^2)
+    if (careful) {
+      irho = 1. / rs;
+      iden = 1. / den;
+    }
+    // Monaghan viscosity for approaching pairs
+    const double nmu = __dmul_rn(__dmul_rn(hij, nvr), iden);
+    const double ac = __dmul_rn(P.alpha_half, __dadd_rn(I.c, r[6].x));
+    const double pi = nvr > 0. ? __dmul_rn(__dmul_rn(fma(P.corr.beta, nmu, ac), nmu), irho) : 0.;
+    a.vt[0] = fma(pi, wx, a.vt[0]);
+    a.vt[1] = fma(pi, wy, a.vt[1]);
+    const double xs = __dmul_rn(w, irho);
+    a.xt[0] = fma(xs, dvx, a.xt[0]);
+    a.xt[1] = fma(xs, dvy, a.xt[1]);
   }
+  // Brookshaw: 2 (m/rho_j)(Ti - Tj)(e_ij . grad W)/r, and (e_ij . grad W)/r = dwr
+  // (at r = 0 the reference leaves the term out: it matters where an operand is not finite)
+  if (I.thermal && (!careful || rr2 > 1e-16)) a.T = fma(__dmul_rn(volj, __dsub_rn(I.T, r[7].x)), dwr, a.T);
 }
 
-__device__ __forceinline__ void pair_fp64_particle(const params &P, const dev_buffers &D, int q) {
-  if (q >= P.N) return;
-  const double *__restrict__ rec = D.rec;
+// The FP64 pair sums of the particles of block bk.x (BS threads, G lanes per particle).
+//
+// Two passes over a particle's window. The first finds its neighbours: the G lanes test the
+// window's candidates (five contiguous ranges, ~56 particles) in FP32 on the 16-byte candidate
+// records, with a margin that keeps every pair of the exact support, STEP candidates a round, and
+// put the ones to take into lists in shared memory (two lanes fill a row from its two ends, so
+// that they share its entries evenly without counting each other's). The second takes the rows'
+// ~30 entries with the FP64 pair term, which tests the support exactly; the lanes' sums are then
+// added in a fixed tree. Rows that fill up are drained before the next round.
+template <int G>
+struct pair64_rows {
+  static constexpr int LANES = G > 1 ? 2 : 1;              // lanes per row
+  static constexpr int STEP = 8;                           // candidates per particle and round
+  static constexpr int U = STEP / G;                       // of which each lane's
+  static constexpr int HALF = G == 1 ? 41 : G == 2 ? 33 : 17;  // entries per lane (rows on distinct banks)
+  static constexpr int CAP = LANES * HALF;
+};
+
+// 4-byte words of the lists of a block of BS threads, whatever the lanes per particle
+template <int BS>
+struct pair64_shared {
+  static constexpr int WORDS = BS * pair64_rows<1>::CAP;
+};
+
+template <int BS, int G>
+__device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffers &D, blk bk, unsigned *s_list) {
+  using R_ = pair64_rows<G>;
+  constexpr int GROUPS = BS / G, U = R_::U, STEP = R_::STEP, LANES = R_::LANES, HALF = R_::HALF, CAP = R_::CAP;
+  static_assert(BS / LANES * CAP <= pair64_shared<BS>::WORDS, "lists fit");
+  const int sub = (int)threadIdx.x & (G - 1), grp = (int)threadIdx.x / G;
+  const int side = (int)threadIdx.x & (LANES - 1);
+  unsigned *const row = s_list + (int)threadIdx.x / LANES * CAP;
+  const int q = bk.x * GROUPS + grp;
   const int N = P.N;
-  double ri[R_WIDTH];
-  load_rec(rec, N, q, ri);
-  const unsigned fi = (unsigned)__double_as_longlong(ri[R_FLAGS]);
-  if (fi & FLAG_BLANKED) return;
-  const bool tool_i = fi & FLAG_TOOL;
-  const bool brookshaw = P.thermal_solver == MF_THERMAL_BROOKSHAW;
-  if (!brookshaw && tool_i) return;  // PSE build: tool particles return early (:160-162)
-
-  const double mass = P.phys.mass;
-  const double wdeltap = P.corr.wdeltap, alpha = P.corr.alpha, beta = P.corr.beta, eta = P.corr.eta;
-  const double eps = P.corr.xspheps;
-  double thermal_alpha = 0.;
-  if (brookshaw) thermal_alpha = !tool_i ? P.trml_wp.alpha : (P.thermal_tool_on ? P.trml_tool.alpha : 0.);
-  const bool thermal = thermal_alpha != 0.;
-
-  const double xi = ri[R_X], yi = ri[R_Y], vxi = ri[R_VX], vyi = ri[R_VY];
-  const double sxxi = ri[R_SXX], sxyi = ri[R_SXY], syyi = ri[R_SYY];
-  const double Rxxi = ri[R_RXX], Rxyi = ri[R_RXY], Ryyi = ri[R_RYY];
-  const double hi = ri[R_H], rhoi = ri[R_RHO], ci = ri[R_C];
-  const double Ti = thermal ? ri[R_T] : 0.;
-  const double h1 = 1 / hi;
-  const double fourh2 = 4 * hi * hi;
-  const bool nonfinite_i = fi & FLAG_NONFINITE;
-
+  const double *__restrict__ rec = D.rec;
+  const float4 *__restrict__ cand = rec_cand(rec, N);
+  const int qc = q < N ? q : N - 1;
+  const float4 ci = __ldg(cand + qc);
+  double2 ri[R_WIDTH / 2];
+#pragma unroll
+  for (int k = 0; k < R_WIDTH / 2; ++k) ri[k] = rec_plane(rec, k, qc);
   const geom g = *D.g;
-  const int hashi = D.hash_cur[q];
-  const int p = __ldg(D.perm + q);  // the start slot (last contact forces), loaded during the sums
-  const int gi = hashi / g.ny;
-  const int gj = hashi - gi * g.ny;
-  const int low_i = gi - 2 < 0 ? 0 : gi - 2;
-  const int low_j = gj - 2 < 0 ? 0 : gj - 2;
-  const int high_i = gi + 3 > g.nx ? g.nx : gi + 3;
-  const int high_j = gj + 3 > g.ny ? g.ny : gj + 3;
+  const int p = __ldg(D.perm + qc);  // the start slot (last contact forces), loaded during the sums
+  const unsigned fi = (unsigned)__double_as_longlong(ri[7].y);
+  const unsigned marks = __float_as_uint(ci.z);
+  const bool any_i = marks & CAND_ANY;
+  const bool brookshaw = P.thermal_solver == MF_THERMAL_BROOKSHAW;
+  pair64_i I;
+  I.tool = fi & FLAG_TOOL;
+  // PSE build: tool particles return early (interactions_gpu.cu:160-162)
+  const bool act = q < N && !(fi & FLAG_BLANKED) && (brookshaw || !I.tool);
+  I.thermal_alpha = 0.;
+  if (brookshaw) I.thermal_alpha = !I.tool ? P.trml_wp.alpha : (P.thermal_tool_on ? P.trml_tool.alpha : 0.);
+  I.thermal = I.thermal_alpha != 0.;
+  I.x = ri[0].x; I.y = ri[0].y; I.vx = ri[1].x; I.vy = ri[1].y;
+  I.sxx = ri[2].x; I.sxy = ri[2].y; I.syy = ri[3].x;
+  I.Rxx = ri[3].y; I.Rxy = ri[4].x; I.Ryy = ri[4].y;
+  I.h = ri[5].x; I.rho = ri[5].y; I.c = ri[6].x; I.T = ri[7].x;
+  I.h1 = any_i ? 1. / I.h : rcp64(I.h);
+  I.fourh2 = 4. * I.h * I.h;
+  I.fac = 0.454728408833987 * I.h1 * I.h1;
+  I.dw_in = -3. * I.h1 * I.h1 * I.fac;
+  I.dw_out = -0.75 * I.h1 * I.fac;
+  pair64_acc a;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) a.v[k] = a.s[k] = 0.;
+  a.vt[0] = a.vt[1] = a.xt[0] = a.xt[1] = a.T = 0.;
 
-  double vdx = 0., vdy = 0., vdz = 0., vdw = 0.;  // v_der
-  double sdx = 0., sdy = 0., sdz = 0., sdw = 0.;  // S_der
-  double vtx = 0., vty = 0., xtx = 0., xty = 0.;   // vel_t (AV), pos_t (XSPH)
-  double T_lapl = 0.;
-
-  const double m_eps = -eps * mass;
-  for (int ii = low_i; ii < high_i; ++ii) {
-    const int j0 = __ldg(D.off + ii * g.ny + low_j);
-    const int j1 = __ldg(D.off + ii * g.ny + high_j);
-    // Candidates are taken in chunks of up to 32: a cheap pass marks the ones that
-    // contribute, then the expensive body visits the marked ones in array order. Outside
-    // the support the reference adds terms multiplied by W = 0: they change no finite sum,
-    // but a NaN/Inf operand turns the sum into NaN, so those candidates are marked too.
-    for (int jb = j0; jb < j1; jb += 32) {
-      const int jn = min(32, j1 - jb);
-      unsigned mask = 0u;
-      for (int k = 0; k < jn; ++k) {
-        const unsigned fj = (unsigned)__double_as_longlong(rec_plane(rec, N, 7, jb + k).y);
-        const double2 xy = rec_plane(rec, N, 0, jb + k);
-        const double xij = xi - xy.x;
-        const double yij = yi - xy.y;
-        const double rr2 = xij * xij + yij * yij;
-        const bool in_support = !(rr2 >= fourh2 || rr2 < 1e-8);
-        const bool take = !(fj & FLAG_BLANKED) && (in_support || nonfinite_i || (fj & FLAG_NONFINITE));
-        mask |= (take ? 1u : 0u) << k;
+  // the test's radius: 2 h with the FP32 positions' error (a few ulp of the cell size) to spare
+  const float dxc = (float)g.dx;
+  const float Rf = 2.00001f * (float)I.h + 1e-5f * dxc;
+  const float R2 = Rf * Rf;
+  const float xi = any_i ? __int_as_float(0x7fffffff) : ci.x;
+  int cnt = 0;
+  auto drain = [&]() {
+    if (LANES > 1) __syncwarp();
+    const int other = LANES > 1 ? __shfl_xor_sync(0xffffffffu, cnt, 1) : 0;
+    const int front = side ? other : cnt, n = cnt + other;  // entries from the row's front, and in all
+    for (int k = side; k < n; k += LANES) {
+      const unsigned e = row[k < front ? k : CAP - 1 - (k - front)];
+      const int j = (int)(e & CAND_COLUMN);
+      double2 r[R_WIDTH / 2];
+#pragma unroll
+      for (int m = 0; m < R_WIDTH / 2; ++m) r[m] = rec_plane(rec, m, j);
+      const bool careful = (e & CAND_ANY) || any_i;
+      // (a blanked candidate gets into a list only when particle i itself takes everything)
+      if (careful && ((unsigned)__double_as_longlong(r[7].y) & FLAG_BLANKED)) continue;
+      pair64_add(P, I, r, e & CAND_TOOL, careful, a);
+    }
+    cnt = 0;
+    if (LANES > 1) __syncwarp();
+  };
+  const int gi = (int)(marks & CAND_COLUMN), gj = (int)ci.w;
+  const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
+  auto bounds = [&](int c, int &j0, int &j1) {  // window column c's particles
+    const int ii = gi - 2 + c;
+    const bool in = act && ii >= 0 && ii < g.nx;
+    j0 = in ? __ldg(D.off + ii * g.ny + low_j) : 0;
+    j1 = in ? __ldg(D.off + ii * g.ny + high_j) : 0;
+  };
+  int n0, n1;
+  bounds(0, n0, n1);
+#pragma unroll 1
+  for (int c = 0; c < 5; ++c) {
+    const int j0 = n0, j1 = n1;
+    if (c < 4) bounds(c + 1, n0, n1);  // the next column's bounds, in flight during this one
+    const float ox = fmaf((float)(2 - c), dxc, xi);
+    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb += STEP) {
+      if (__any_sync(0xffffffffu, cnt > HALF - U)) drain();
+      float4 b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = jb + u * G + sub;
+        b[u] = __ldg(cand + (j < j1 ? j : qc));
       }
-      while (mask) {
-        const int k = __ffs(mask) - 1;
-        mask &= mask - 1u;
-        const int j = jb + k;
-        const double2 fx = rec_plane(rec, N, 7, j);    // T, flags
-        const double2 xy = rec_plane(rec, N, 0, j);
-        const double2 cvol = rec_plane(rec, N, 6, j);  // c, vol
-        const unsigned fj = (unsigned)__double_as_longlong(fx.y);
-        const double xij = xi - xy.x;
-        const double yij = yi - xy.y;
-        const double rr2 = xij * xij + yij * yij;
-        const bool in_support = !(rr2 >= fourh2 || rr2 < 1e-8);
-        double w = 0., w_x = 0., w_y = 0., dwr = 0.;
-        if (in_support) cubic_spline_fp64(xij, yij, rr2, h1, w, w_x, w_y, dwr);
-        const double volj = cvol.y;
-        const bool tool_j = fj & FLAG_TOOL;
-        if (!tool_i && !tool_j) {
-          const double2 v = rec_plane(rec, N, 1, j);
-          const double2 s01 = rec_plane(rec, N, 2, j);   // sxx, sxy
-          const double2 s2r0 = rec_plane(rec, N, 3, j);  // syy, Rxx
-          const double2 r12 = rec_plane(rec, N, 4, j);   // Rxy, Ryy
-          const double2 hrho = rec_plane(rec, N, 5, j);  // h, rho
-          vdx += (v.x - vxi) * w_x * volj;
-          vdy += (v.x - vxi) * w_y * volj;
-          vdz += (v.y - vyi) * w_x * volj;
-          vdw += (v.y - vyi) * w_y * volj;
-          double fab = w / wdeltap;
-          fab *= fab;
-          fab *= fab;
-          const double Rx = fab * (Rxxi + s2r0.y);
-          const double Ry = fab * (Rxyi + r12.x);
-          const double Rz = fab * (Ryyi + r12.y);
-          sdx += mass * (sxxi + s01.x + Rx) * w_x;
-          sdy += mass * (sxyi + s01.y + Ry) * w_y;
-          sdz += mass * (sxyi + s01.y + Ry) * w_x;
-          sdw += mass * (syyi + s2r0.x + Rz) * w_y;
-          const double vijx = vxi - v.x;
-          const double vijy = vyi - v.y;
-          const double vijposij = vijx * xij + vijy * yij;
-          const double irhoij = 1. / (0.5 * (rhoi + hrho.y));
-          if (vijposij < 0.) {
-            const double cij = 0.5 * (ci + cvol.x);
-            const double hij = 0.5 * (hi + hrho.x);
-            const double muij = (hij * vijposij) / (rr2 + eta * eta * hij * hij);
-            const double piij = (-alpha * cij * muij + beta * muij * muij) * irhoij;
-            vtx += -mass * piij * w_x;
-            vty += -mass * piij * w_y;
-          }
-          const double xs = m_eps * w * irhoij;
-          xtx += xs * vijx;
-          xty += xs * vijy;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = jb + u * G + sub;
+        const float xij = ox - b[u].x;
+        const float yij = fmaf(ci.w - b[u].w, dxc, ci.y - b[u].y);
+        const float rr2 = fmaf(xij, xij, yij * yij);
+        if (j < j1 && !(rr2 > R2) && (j != q || any_i)) {
+          row[side ? CAP - 1 - cnt : cnt] = (unsigned)j | (__float_as_uint(b[u].z) & (CAND_TOOL | CAND_ANY));
+          ++cnt;
         }
-        // Brookshaw: 2 (m/rho_j)(Ti - Tj)(e_ij . grad W)/r, and (e_ij . grad W)/r = der*fac
-        if (thermal && rr2 > 1e-16) T_lapl += 2.0 * volj * (Ti - fx.x) * dwr;
       }
     }
   }
-
+  drain();
+  // the lanes' sums, in a fixed tree; every lane holds the total
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a.v[k] += __shfl_xor_sync(0xffffffffu, a.v[k], o);
+      a.s[k] += __shfl_xor_sync(0xffffffffu, a.s[k], o);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      a.vt[k] += __shfl_xor_sync(0xffffffffu, a.vt[k], o);
+      a.xt[k] += __shfl_xor_sync(0xffffffffu, a.xt[k], o);
+    }
+    a.T += __shfl_xor_sync(0xffffffffu, a.T, o);
+  }
+  if (!act) return;
+  // the rates (actions_gpu.cu:99-224), shared out over the particle's lanes
   const state_set &B = D.B;
-  if (P.keep_derivs) {
-    D.S_der[q] = make_double4(sdx, sdy, sdz, sdw);
-    D.v_der[q] = make_double4(vdx, vdy, vdz, vdw);
+  const double mass = P.phys.mass;
+  const double sdx = __dmul_rn(mass, a.s[0]), sdy = __dmul_rn(mass, a.s[1]);
+  const double sdz = __dmul_rn(mass, a.s[2]), sdw = __dmul_rn(mass, a.s[3]);
+  if (sub == 0) {
+    if (P.keep_derivs) {
+      D.S_der[q] = make_double4(sdx, sdy, sdz, sdw);
+      D.v_der[q] = make_double4(a.v[0], a.v[1], a.v[2], a.v[3]);
+    }
+    if (!I.tool) {
+      const double4 S = B.S[q];  // predicted stress
+      double tx, ty, tz, tw;
+      jaumann(P.phys.G, a.v[0], a.v[1], a.v[2], a.v[3], S.x, S.y, S.z, S.w, tx, ty, tz, tw);
+      B.S_t[q] = make_double4(tx, ty, tz, tw);
+      B.rho_t[q] = -I.rho * (a.v[0] + a.v[3]);
+    }
   }
-  if (!tool_i) {
-    const double4 S = B.S[q];  // predicted stress
-    double tx, ty, tz, tw;
-    jaumann(P.phys.G, vdx, vdy, vdz, vdw, S.x, S.y, S.z, S.w, tx, ty, tz, tw);
-    B.S_t[q] = make_double4(tx, ty, tz, tw);
-    B.rho_t[q] = -rhoi * (vdx + vdw);
-    double2 fc, ft;
-    prev_contact_forces(P, D, q, p, fc, ft);
-    double2 vel_t;
-    vel_t.x = vtx + (sdx + sdy + fc.x / mass + ft.x / mass);
-    vel_t.y = vty + (sdz + sdw + fc.y / mass + ft.y / mass);
+  if (sub == (G > 1 ? 1 : 0)) {
+    const double m2 = 2. * mass, m_eps = __dmul_rn(P.corr.xspheps, m2);
+    double2 vel_t = make_double2(__dmul_rn(-m2, a.vt[0]), __dmul_rn(-m2, a.vt[1]));
+    double2 pos_t = make_double2(__dmul_rn(m_eps, a.xt[0]), __dmul_rn(m_eps, a.xt[1]));
+    if (!I.tool) {
+      double2 fc, ft;
+      prev_contact_forces(P, D, q, p, fc, ft);
+      double ax = __dadd_rn(sdx, sdy), ay = __dadd_rn(sdz, sdw);
+      if (fc.x != 0. || fc.y != 0. || ft.x != 0. || ft.y != 0.) {
+        ax = __dadd_rn(ax, __dadd_rn(fc.x / mass, ft.x / mass));
+        ay = __dadd_rn(ay, __dadd_rn(fc.y / mass, ft.y / mass));
+      }
+      vel_t = make_double2(__dadd_rn(vel_t.x, ax), __dadd_rn(vel_t.y, ay));
+      pos_t = make_double2(__dadd_rn(pos_t.x, I.vx), __dadd_rn(pos_t.y, I.vy));
+    }
     B.vel_t[q] = vel_t;
-    B.pos_t[q] = make_double2(xtx + vxi, xty + vyi);
-  } else {
-    B.vel_t[q] = make_double2(vtx, vty);
-    B.pos_t[q] = make_double2(xtx, xty);
+    B.pos_t[q] = pos_t;
+    if (I.thermal) B.T_t[q] = I.thermal_alpha * (2. * a.T);
   }
-  if (thermal) B.T_t[q] = thermal_alpha * T_lapl;
 }
 
-// the FP64 pair sums of block bk.x's particles
-__device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffers &D, blk bk) {
-  pair_fp64_particle(P, D, bk.x * blockDim.x + threadIdx.x);
-}
+// Lanes per particle: as many as still let every particle's lanes be resident at once (16 warps
+// per SM on 148 SMs: 18,944 particles at 4, 37,888 at 2), then one. A small system's time is one
+// particle's chain of neighbours, which more lanes shorten; a large one's is the work, of which
+// every lane repeats the particle's share (record, window, rates). Pair stage in us (launch
+// included) at 1 / 2 / 4 lanes: 7,096 particles 25.6 / 19.5 / 17.4; 16,800 25.6 / 19.5 / 17.4;
+// 23,416 26.6 / 21.5 / 25.6; 31,261 27.6 / 23.6 / 29.7; 45,052 29.7 / 33.8 / 35.8;
+// 70,316 35.8 / 39.9 / 50.2; 176,695 78.8 / 87.0 / 111.6; 577,555 220 / 261 / 345.
+// (One thread per particle over the window in FP64, without the lists: 45, -, 58 at 32,468, 123
+// at 176,695.) The lanes decide the order of a particle's sums, so the rule looks at the system's
+// own size only: a system in a batch gives the bits it gives by itself.
+__host__ __device__ constexpr int pair64_lanes(int N) { return N <= 18944 ? 4 : N <= 37888 ? 2 : 1; }
 
-// the FP64 pair kernel in blocks of 64 at 8 per SM (128 registers): 110.6 against 112.6 us in
-// blocks of 128 at 4, 114.7 in blocks of 256 at 2 (the ~150k-particle cut); at 3 blocks of 128
-// (153 registers, no spills) 121.8
+// 64-thread blocks at 8 per SM (128 registers, no spills). At 10 per SM (96 registers, 150 B of
+// spills) 121 against 86 us for the ~177k-particle cut at 2 lanes, at 7 per SM 91.
 constexpr int PAIR64_BLOCK = 64;
-#ifndef MF_PAIR64_MIN_BLOCKS
-#define MF_PAIR64_MIN_BLOCKS 8
-#endif
-static __global__ void __launch_bounds__(PAIR64_BLOCK, MF_PAIR64_MIN_BLOCKS) k_pair_fp64(params P, dev_buffers D) {
+template <int G>
+static __global__ void __launch_bounds__(PAIR64_BLOCK, 8) k_pair_fp64(params P, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
-  pair_fp64_body(P, D, grid_blk());
+  __shared__ unsigned s_list[PAIR64_BLOCK / pair64_rows<G>::LANES * pair64_rows<G>::CAP];
+  pair_fp64_body<PAIR64_BLOCK, G>(P, D, grid_blk(), s_list);
 }
 
 // PSE heat Laplacian (interactions_gpu.cu:88-144): every particle of the window, blanked
@@ -822,11 +974,11 @@ __device__ __forceinline__ void pse_body(const params &P, const dev_buffers &D, 
   if (q >= P.N) return;
   const double *__restrict__ rec = D.rec;
   const int N = P.N;
-  const double2 fx = rec_plane(rec, N, 7, q);
+  const double2 fx = rec_plane(rec, 7, q);
   const unsigned fi = (unsigned)__double_as_longlong(fx.y);
   if (fi & FLAG_BLANKED) return;
-  const double2 xy = rec_plane(rec, N, 0, q);
-  const double hi = rec_plane(rec, N, 5, q).x;
+  const double2 xy = rec_plane(rec, 0, q);
+  const double hi = rec_plane(rec, 5, q).x;
   const double Ti = fx.x;
   const double mass = P.phys.mass;
   const long long tex_elems = ((long long)sizeof(int) * P.N) / 8;
@@ -845,9 +997,9 @@ __device__ __forceinline__ void pse_body(const params &P, const dev_buffers &D, 
     const int j0 = __ldg(D.off + ii * g.ny + low_j);
     const int j1 = __ldg(D.off + ii * g.ny + high_j);
     for (int j = j0; j < j1; ++j) {
-      const double2 pj = rec_plane(rec, N, 0, j);
-      const double Tj = rec_plane(rec, N, 7, j).x;
-      const double rhoj = rec_plane(rec, N, 5, j).y;
+      const double2 pj = rec_plane(rec, 0, j);
+      const double Tj = rec_plane(rec, 7, j).x;
+      const double rhoj = rec_plane(rec, 5, j).y;
       const double w2 = lapl_pse_fp64(xy.x - pj.x, xy.y - pj.y, hi);
       T_ti += (Tj - Ti) * w2 * mass / rhoj;
     }
