@@ -17,6 +17,7 @@
 #include "mf_mixed.cuh"
 #include "mf_batch.cuh"
 #include "mf_persist.h"
+#include "mf_tangent.h"
 #include "mfree_b200.h"
 
 using namespace mf;
@@ -31,19 +32,6 @@ struct nvtx_range {
   nvtx_range &operator=(const nvtx_range &) = delete;
 };
 }  // namespace
-
-namespace mf {
-// the differentiable step (csrc/mf_tangent.cu): one derivative direction (tg), all six (tg6);
-// out_dmean holds d(mean Fc), d(mean Ff) per direction
-namespace tg {
-int run_mean_force(mf_ctx *ctx, int device, params P, const dev_buffers &Dctx, int skip_steps, int window_steps,
-                   int param, double out_mean[2], double out_dmean[]);
-}  // namespace tg
-namespace tg6 {
-int run_mean_force(mf_ctx *ctx, int device, params P, const dev_buffers &Dctx, int skip_steps, int window_steps,
-                   int param, double out_mean[2], double out_dmean[]);
-}  // namespace tg6
-}  // namespace mf
 
 // one asynchronous particle dump: a device snapshot of the fields, their copy into pinned
 // host memory on a side stream, and a host thread that writes the file once it has landed
@@ -98,6 +86,7 @@ struct mf_ctx {
   long long steps = 0;
   unsigned long long force_read_head = 0;
   unsigned long long status_newly_blanked_seen = 0;
+  tg::workspace tangent;  // the differentiable step's memory, kept between its calls
   cudaStream_t io_stream = nullptr;  // device-to-host copies of asynchronous dumps
   std::vector<std::unique_ptr<vtk_job>> vtk_jobs;
 };
@@ -183,6 +172,7 @@ int invalidate_counts(mf_ctx *ctx) {
 int alloc_particles(mf_ctx *ctx, int N) {
   drop_graphs(ctx);
   free_list(ctx->particle_allocs);
+  tg::release(ctx->tangent);
   auto &L = ctx->particle_allocs;
   TRY(alloc_set(ctx, ctx->set[0], N));
   TRY(alloc_set(ctx, ctx->set[1], N));
@@ -558,6 +548,7 @@ int mf_ctx_destroy(mf_ctx *ctx) {
   if (ctx->io_stream) cudaStreamDestroy(ctx->io_stream);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   drop_graphs(ctx);
+  tg::release(ctx->tangent);
   free_list(ctx->particle_allocs);
   free_list(ctx->grid_allocs);
   free_list(ctx->fixed_allocs);
@@ -1963,28 +1954,37 @@ int tangent_check(mf_ctx *ctx) {
 }
 }  // namespace
 
+namespace {
+int tangent_run(mf_ctx *ctx, int skip_steps, int window_steps, const int *dirs, int n, double *out_mean,
+                double *out_dmean) {
+  TRY(tangent_check(ctx));
+  TRY(set_device(ctx));
+  mf_tool_state tool;
+  TRY(mf_tool_get(ctx, &tool));
+  params P = ctx->P;
+  P.N = ctx->N;
+  return tg::run_mean_force(P, ctx->D, ctx->set[ctx->cur], tool, ctx->G.max_cell, ctx->stream, ctx->tangent,
+                            skip_steps, window_steps, dirs, n, out_mean, out_dmean, &ctx->last_cuda_err);
+}
+}  // namespace
+
 int mf_tangent_mean_force_all(mf_ctx *ctx, int skip_steps, int window_steps, double out_mean[2],
                               double out_dmean[12]) {
   nvtx_range range("mf_tangent_mean_force_all");
   if (!ctx || !out_mean || !out_dmean || skip_steps < 0 || window_steps < 1) return MF_ERR_INVALID;
-  TRY(tangent_check(ctx));
-  TRY(set_device(ctx));
-  CK(cudaStreamSynchronize(ctx->stream));
-  params P = ctx->P;
-  P.N = ctx->N;
-  P.staged = 0;
-  return mf::tg6::run_mean_force(ctx, ctx->device, P, ctx->D, skip_steps, window_steps, -1, out_mean, out_dmean);
+  const int dirs[6] = {0, 1, 2, 3, 4, 5};
+  return tangent_run(ctx, skip_steps, window_steps, dirs, 6, out_mean, out_dmean);
 }
 
 int mf_tangent_mean_force(mf_ctx *ctx, int skip_steps, int window_steps, int param, double out_mean[2],
                           double out_dmean[2]) {
   nvtx_range range("mf_tangent_mean_force");
   if (!ctx || !out_mean || skip_steps < 0 || window_steps < 1 || param < -1 || param > 5) return MF_ERR_INVALID;
-  TRY(tangent_check(ctx));
-  TRY(set_device(ctx));
-  CK(cudaStreamSynchronize(ctx->stream));
-  params P = ctx->P;
-  P.N = ctx->N;
-  P.staged = 0;
-  return mf::tg::run_mean_force(ctx, ctx->device, P, ctx->D, skip_steps, window_steps, param, out_mean, out_dmean);
+  double dmean[2] = {0., 0.};
+  TRY(tangent_run(ctx, skip_steps, window_steps, &param, param >= 0 ? 1 : 0, out_mean, dmean));
+  if (out_dmean) {
+    out_dmean[0] = dmean[0];
+    out_dmean[1] = dmean[1];
+  }
+  return MF_OK;
 }
