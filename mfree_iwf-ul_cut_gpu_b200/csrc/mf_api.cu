@@ -178,8 +178,9 @@ int alloc_particles(mf_ctx *ctx, int N) {
   TRY(alloc_set(ctx, ctx->set[1], N));
   dev_buffers &D = ctx->D;
   TRY(dalloc(ctx, L, &D.n, N));
-  TRY(dalloc(ctx, L, &D.rec, rec_doubles(N) + (size_t)N * 2));  // pair records, candidate records
-  TRY(dalloc(ctx, L, &D.recf, (size_t)N * F_WIDTH));
+  TRY(dalloc(ctx, L, &D.rec, rec_doubles(N) + ((size_t)N + CAND_PAD) * 2));  // pair records, candidate records
+  TRY(dalloc(ctx, L, &D.recf, recf_floats(N)));
+  TRY(dalloc(ctx, L, &D.col, N));
   TRY(dalloc(ctx, L, &D.S_der, N));
   TRY(dalloc(ctx, L, &D.v_der, N));
   TRY(dalloc(ctx, L, &D.hash_cur, N));
@@ -324,6 +325,16 @@ int launch_pair_fp64(mf_ctx *ctx) {
   }
 }
 
+template <bool LIST>
+int launch_pair_mixed(mf_ctx *ctx) {
+  const int lanes = mixed_parts(ctx->N), per = PAIR_BLOCK / lanes, nb = (ctx->N + per - 1) / per;
+  switch (lanes) {
+    case 4: return launch_pdl(ctx, k_pair_mixed<4, LIST>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    case 2: return launch_pdl(ctx, k_pair_mixed<2, LIST>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    default: return launch_pdl(ctx, k_pair_mixed<1, LIST>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+  }
+}
+
 int launch_stage(mf_ctx *ctx, int stage) {
   static const char *const names[4] = {"mf stage 0: cell list", "mf stage 1: predictor",
                                        "mf stage 2: pair sums", "mf stage 3: finish + return map"};
@@ -343,8 +354,7 @@ int launch_stage(mf_ctx *ctx, int stage) {
       else TRY(launch_pdl(ctx, k_reorder<true, false>, nb, BLOCK, ctx->P, ctx->D));
       break;
     case 2:
-      if (mixed && ctx->P.verlet) TRY(launch_pdl(ctx, k_pair_mixed<true>, npb, PAIR_BLOCK, ctx->P, ctx->D));
-      else if (mixed) TRY(launch_pdl(ctx, k_pair_mixed<false>, npb, PAIR_BLOCK, ctx->P, ctx->D));
+      if (mixed) TRY(ctx->P.verlet ? launch_pair_mixed<true>(ctx) : launch_pair_mixed<false>(ctx));
       else TRY(launch_pair_fp64(ctx));
       if (ctx->P.thermal_solver == MF_THERMAL_PSE && ctx->P.thermal_wp) {
         if (mixed) TRY(launch_pdl(ctx, k_pse_mixed, npb, PAIR_BLOCK, ctx->P, ctx->D));
@@ -692,8 +702,8 @@ int mf_get_field(mf_ctx *ctx, int field, void *host) {
     double *o = (double *)host;
     if (ctx->P.precision == MF_PRECISION_MIXED && !ctx->last_staged) {
       // mixed form: R lives only in the FP32 pair records
-      std::vector<float> rec(N * F_WIDTH);
-      CK(cudaMemcpy(rec.data(), ctx->D.recf, sizeof(float) * N * F_WIDTH, cudaMemcpyDeviceToHost));
+      std::vector<float> rec(recf_floats((int)N));
+      CK(cudaMemcpy(rec.data(), ctx->D.recf, sizeof(float) * rec.size(), cudaMemcpyDeviceToHost));
       for (size_t i = 0; i < N; ++i) {
         auto at = [&](int f) { return rec[recf_word(f / 4, (int)i, (int)N) * 4 + f % 4]; };
         o[4 * i] = at(F_RXX);

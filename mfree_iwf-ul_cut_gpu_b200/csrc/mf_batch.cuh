@@ -99,13 +99,24 @@ static __global__ void __launch_bounds__(BS) kb_pair_fp64(batch_map M) {
   }
 }
 
+// the mixed pair sums of a system's block, in the parts of the system's size, at one lane per particle
+template <int BS>
+__device__ __forceinline__ void pair_mixed_system(const params &P, const dev_buffers &D, blk b, unsigned *s_list) {
+  switch (mixed_parts(P.N)) {
+    case 4: pair_mixed_body<BS, 1, 4, false>(P, D, b, s_list); break;
+    case 2: pair_mixed_body<BS, 1, 2, false>(P, D, b, s_list); break;
+    default: pair_mixed_body<BS, 1, 1, false>(P, D, b, s_list); break;
+  }
+}
+
 template <int BS>
 static __global__ void __launch_bounds__(BS, 640 / BS) kb_pair_mixed(batch_map M) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  pair_mixed_body<false>(s.P, s.D, b);
+  __shared__ unsigned s_list[mixed_shared<BS>::WORDS];
+  pair_mixed_system<BS>(s.P, s.D, b, s_list);
 }
 
 template <int BS>

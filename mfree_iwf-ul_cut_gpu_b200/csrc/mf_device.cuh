@@ -27,19 +27,30 @@ enum : int {
 };
 
 // FP32 pair record of the mixed form (16 floats = 64 bytes): coordinates relative to the
-// origin of the particle's own cell; the first 16 bytes (x, y, flags | cell_y << 8, vx) are
-// all the distance test needs
+// origin of the particle's own cell. The first 16 bytes are all the distance test needs; its last
+// two floats carry the marks: F_ROW is the cell's row + 1, negative for a tool particle and NaN for
+// a blanked one (so that no distance test takes it), F_H the smoothing length, negative when the
+// record holds a NaN or Inf. The order lets a pair's packed operands be neighbours in a word.
 enum : int {
-  F_X = 0, F_Y, F_FLAGS, F_VX, F_VY, F_SXX, F_SXY, F_SYY, F_RXX, F_RXY, F_RYY, F_H, F_RHO, F_C, F_VOL, F_T,
+  F_X = 0, F_Y, F_ROW, F_H, F_VX, F_VY, F_SXY, F_RXY, F_SXX, F_SYY, F_RXX, F_RYY, F_RHO, F_C, F_VOL, F_T,
   F_WIDTH
 };
 
-// index of float4 word k (0..3) of particle j's FP32 pair record among N records: four planes,
-// word k of every particle together at k N + j. (Each particle's 64 bytes together, at 4 j + k,
-// measured 68 % slower in the list pair kernel: a warp's 16-byte loads then touch four times as
-// many cache lines, and L1 throughput becomes the limit.)
+// candidates a search may read past the last one (whole rounds are loaded, what lies beyond is
+// not used): the arrays of candidate records are that much longer
+constexpr int CAND_PAD = 8;
+// index of float4 word k (0..3) of particle j's FP32 pair record among N records: word 0, what the
+// distance test reads, of all particles together; the others in tiles of 32 particles, word k of a
+// tile's particles together (512 bytes), so that a warp's loads of one word are coalesced and one
+// address serves the three (constant offsets). (Each particle's 64 bytes together measured
+// 68 % slower in the list pair kernel: a warp's 16-byte loads then touch four times as many cache
+// lines, and L1 throughput becomes the limit.)
 __host__ __device__ __forceinline__ size_t recf_word(int k, int j, int N) {
-  return (size_t)k * (size_t)N + (size_t)j;
+  constexpr int W = F_WIDTH / 4 - 1;
+  return k == 0 ? (size_t)j : (size_t)N + CAND_PAD + (size_t)(j >> 5) * (W * 32) + (size_t)((k - 1) * 32 + (j & 31));
+}
+__host__ __device__ __forceinline__ size_t recf_floats(int N) {
+  return ((size_t)N + CAND_PAD) * 4 + (size_t)((N + 31) / 32) * 32 * (F_WIDTH - 4);
 }
 
 struct params {

@@ -49,8 +49,9 @@ struct plastic_item {
 struct dev_buffers {
   state_set A, B;       // A: state at the start of the step (previous order), B: new order
   double2 *n;           // contact normal, indexed by array position (never permuted)
-  double *rec;          // FP64 pair records: R_WIDTH / 2 planes of N double2
-  float *recf;          // FP32 pair records (mixed form): F_WIDTH / 4 planes of N float4
+  double *rec;          // FP64 pair records (rec_word) and candidate records (rec_cand)
+  float *recf;          // FP32 pair records (mixed form), recf_word
+  int *col;             // mixed form: column of the particle's cell
   double4 *S_der, *v_der;
   int *hash_cur;        // cell hash per array position (sorted order)
   int *hash_new, *perm;
@@ -455,6 +456,7 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
   B.pp[q] = prs;
   unsigned rf = f & (FLAG_BLANKED | FLAG_TOOL | FLAG_FIXED);
   float fr[F_WIDTH];
+  constexpr int fk[12] = {F_VX, F_VY, F_SXX, F_SXY, F_SYY, F_RXX, F_RXY, F_RYY, F_H, F_RHO, F_C, F_VOL};
   if (!MIXED || P.staged) {
     double Rxx = 0., Rxy = 0., Ryy = 0.;
     if (!tool) artificial_stress(rho, prs, S.x, S.y, S.z, P.corr.stresseps, Rxx, Rxy, Ryy);
@@ -485,7 +487,7 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     const float fv[12] = {(float)vel.x, (float)vel.y, (float)sxx, (float)sxy, (float)syy, (float)Rxx,
                           (float)Rxy, (float)Ryy, (float)h, (float)rho, (float)c, (float)vol};
 #pragma unroll
-    for (int k = 0; k < 12; ++k) fr[3 + k] = fv[k];
+    for (int k = 0; k < 12; ++k) fr[fk[k]] = fv[k];
   } else {
     // the mixed form's FP32 record only: one FP64 reciprocal of rho for 1 / rho^2, c and the
     // volume, the artificial stress in float
@@ -498,7 +500,7 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     bool finite = isfinite(pos.x) && isfinite(pos.y) && isfinite(T);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      fr[3 + k] = fv[k];
+      fr[fk[k]] = fv[k];
       finite = finite && isfinite(fv[k]);
     }
     if (!finite) rf |= FLAG_NONFINITE;
@@ -510,11 +512,12 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     const geom g = *D.g;
     const int ci = hsh / g.ny, cj = hsh - ci * g.ny;
     const double ox = g.bbmin_x + ci * g.dx, oy = g.bbmin_y + cj * g.dx;
-    fr[0] = (float)(pos.x - ox);
-    fr[1] = (float)(pos.y - oy);
-    fr[2] = __int_as_float((int)(rf | ((unsigned)cj << 8)));
-    fr[15] = (float)(T - P.trml_wp.T_init);
-    // four float4 words (recf_word: four planes, or each record's words together)
+    fr[F_X] = (float)(pos.x - ox);
+    fr[F_Y] = (float)(pos.y - oy);
+    fr[F_ROW] = blanked ? __int_as_float(0x7fffffff) : tool ? -(float)(cj + 1) : (float)(cj + 1);
+    if (rf & FLAG_NONFINITE) fr[F_H] = __uint_as_float(__float_as_uint(fr[F_H]) | 0x80000000u);
+    fr[F_T] = (float)(T - P.trml_wp.T_init);
+    D.col[q] = ci;
     float4 *fd = reinterpret_cast<float4 *>(D.recf);
 #pragma unroll
     for (int k = 0; k < F_WIDTH / 4; ++k)
@@ -872,8 +875,7 @@ __device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffer
       float4 b[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int j = jb + u * G + sub;
-        b[u] = __ldg(cand + (j < j1 ? j : qc));
+        b[u] = __ldg(cand + (jb + u * G + sub));  // (past the column's end: not used)
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {

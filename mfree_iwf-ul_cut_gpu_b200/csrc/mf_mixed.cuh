@@ -17,151 +17,176 @@
 
 namespace mf {
 
+// the marks in a record's first word (F_ROW, F_H)
+__device__ __forceinline__ bool f_blanked(const float4 &b0) { return b0.z != b0.z; }
+__device__ __forceinline__ bool f_tool(const float4 &b0) { return __float_as_int(b0.z) < 0; }
+__device__ __forceinline__ bool f_nonfinite(const float4 &b0) { return __float_as_int(b0.w) < 0; }
+
 // the i particle's values and the pair sums of one thread
 struct mixed_i {
-  float x, y, sxy, Rxy, h, rho, c, T;
-  float2 nv;      // (-vx, -vy)
-  float2 s_diag;  // (sxx, syy)
-  float2 r_diag;  // (Rxx, Ryy)
-  float h1, fourh2, fac;
+  float x, y, row, vx, vy, sxx, sxy, syy, Rxx, Rxy, Ryy, h, rho, c, T;  // row: cell row + 1
+  float h1, fourh2;
+  // the spline's coefficients: W / W(dp) for q > 1 (w_out (2 - q)^6) and q <= 1 (w_in (1 - 1.5 q^2 +
+  // 0.75 q^3)), (dW/dr) / r for q > 1 (d_out (2 - q)^2 / r) and q <= 1 (d_in (1 - 0.75 q))
+  float w_out, w_in, d_out, d_in;
   bool mech, thermal, nonfinite;
 };
-// Lane pairs for the packed FP32 instructions of sm_100 (two FMAs per issue). The constant
-// factors of a sum are applied once at the end: the stress and viscosity sums without the
-// mass, XSPH without mass * eps, the Brookshaw sum without its factor 2.
+// The constant factors of a sum are applied once at the end: the stress sums without the mass, the
+// viscosity sums without -2 mass, XSPH without 2 mass eps W(dp), the Brookshaw sum without its factor 2.
 struct mixed_acc {
-  float2 vd01, vd23;  // (vdx, vdy), (vdz, vdw)
-  float2 sd_xw;       // (sdx, sdw) / mass
-  float2 sd_zy;       // (sdz, sdy) / mass
-  float2 vt;          // (vtx, vty) / mass
-  float2 xt;          // (xtx, xty) / (mass * eps)
-  float T_lapl;       // / 2
+  float vdx, vdy, vdz, vdw;
+  float sdx, sdy, sdz, sdw;
+  float vtx, vty, xtx, xty;
+  float T_lapl;
 };
 struct mixed_const {
-  float inv_wdeltap, alpha, beta, eta2;
+  float alpha4, beta4, eta4;  // alpha / 4, beta / 4, eta^2 / 4
 };
 
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
 // r^2 with its one fused multiply-add written out, so that every kernel that tests or uses a
-// pair's distance (window, list build, list) rounds it the same way: the list form and the
-// window form then give the same sums bit for bit on a step that builds the lists
+// pair's distance (window, list build, list) rounds it the same way
 __device__ __forceinline__ float dist2(float x, float y) { return fmaf(x, x, __fmul_rn(y, y)); }
+// offset of a record's particle from particle i, dcol columns of cells (i's - j's) and the rows'
+// difference away: the in-cell offsets' difference first, then one rounding
+__device__ __forceinline__ float offset_x(const mixed_i &I, const float4 &b0, float dcol, float dxc) {
+  return fmaf(dcol, dxc, I.x - b0.x);
+}
+__device__ __forceinline__ float offset_y(const mixed_i &I, const float4 &b0, float dxc) {
+  return fmaf(I.row - fabsf(b0.z), dxc, I.y - b0.y);
+}
 
-// one neighbour j (records b0..b3) of particle i at offset (xij, yij)
+// One neighbour j (records b0..b3) of particle i at offset (xij, yij): the reference's cubic spline
+// (kernels.cuh:30-70; its value (2 - q)^6 / 4 for q > 1 is sic), both branches evaluated and selected,
+// with the constants folded into the coefficients (1 / r cancels for q <= 1). In scalars, every
+// multiply-add written out: sm_100's packed pairs (two multiply-adds an issue) save issues only where
+// both operands already lie in register pairs; the moves that built pairs of duplicated factors cost
+// the ALU pipe more than the packed arithmetic gave back (1,100 against 1,770 integer instructions a
+// particle at ~577k particles).
+template <bool SELECT>
 __device__ __forceinline__ void mixed_interact(const mixed_i &I, const mixed_const &K, mixed_acc &a, float xij,
                                                float yij, const float4 &b0, const float4 &b1, const float4 &b2,
                                                const float4 &b3) {
-  const unsigned fjw = (unsigned)__float_as_int(b0.z);
   const float rr2 = dist2(xij, yij);
+  // outside the support (candidates taken because a record holds a NaN or Inf) W = 0
   const bool in_support = !(rr2 >= I.fourh2 || rr2 < 1e-8f);
-  // the reference's cubic spline (kernels.cuh:30-70), its value (2 - q)^6 / 4 for q > 1 (sic:
-  // _2mq2 cubed) included. (Evaluating both branches and selecting, to keep a warp's lanes
-  // together, measured 8 us slower on the ~150k-particle cut.)
-  float w = 0.f, dwr = 0.f;
-  if (in_support) {
-    const float rinv = rsqrtf(rr2);
-    const float qq = rr2 * rinv * I.h1;
-    float val, der;
-    if (qq > 1.f) {
-      const float t = 2.f - qq;
-      const float t2 = t * t;
-      val = 0.25f * t2 * t2 * t2;
-      der = -0.75f * t2 * I.h1 * rinv;
+  float w = 0.f, dwr = 0.f;  // W / W(dp), (dW/dr) / r
+  auto kernel = [&](float rinv) {
+    const float qq = __fmul_rn(__fmul_rn(rr2, rinv), I.h1);
+    const float t = 2.f - qq, t2 = __fmul_rn(t, t);
+    if (SELECT) {
+      const float val_out = __fmul_rn(__fmul_rn(t2, t2), __fmul_rn(I.w_out, t2));
+      const float val_in = __fmul_rn(I.w_in, fmaf(__fmul_rn(qq, qq), fmaf(0.75f, qq, -1.5f), 1.f));
+      const float der_out = __fmul_rn(__fmul_rn(I.d_out, t2), rinv);
+      const float der_in = __fmul_rn(I.d_in, fmaf(-0.75f, qq, 1.f));
+      w = qq > 1.f ? val_out : val_in;
+      dwr = qq > 1.f ? der_out : der_in;
+    } else if (qq > 1.f) {
+      w = __fmul_rn(__fmul_rn(t2, t2), __fmul_rn(I.w_out, t2));
+      dwr = __fmul_rn(__fmul_rn(I.d_out, t2), rinv);
     } else {
-      val = fmaf(-1.5f * qq * qq, fmaf(-0.5f, qq, 1.f), 1.f);
-      der = -3.0f * qq * fmaf(-0.75f, qq, 1.f) * I.h1 * rinv;
+      w = __fmul_rn(I.w_in, fmaf(__fmul_rn(qq, qq), fmaf(0.75f, qq, -1.5f), 1.f));
+      dwr = __fmul_rn(I.d_in, fmaf(-0.75f, qq, 1.f));
     }
-    w = val * I.fac;
-    dwr = der * I.fac;
-  }
-  const float2 pij = f2(xij, yij);
-  const float2 w_xy = __fmul2_rn(f2(dwr, dwr), pij);
+  };
+  if (in_support) kernel(rsqrtf(rr2));
+  const float wx = __fmul_rn(dwr, xij), wy = __fmul_rn(dwr, yij);
   const float volj = b3.z;
-  if (I.mech && !(fjw & FLAG_TOOL)) {
-    const float2 dv = __fadd2_rn(f2(b0.w, b1.x), I.nv);
-    const float2 av = __fmul2_rn(dv, f2(volj, volj));
-    a.vd01 = __ffma2_rn(f2(av.x, av.x), w_xy, a.vd01);
-    a.vd23 = __ffma2_rn(f2(av.y, av.y), w_xy, a.vd23);
-    float fab = w * K.inv_wdeltap;
-    fab *= fab;
-    fab *= fab;
-    const float2 sd = __ffma2_rn(f2(fab, fab), __fadd2_rn(I.r_diag, f2(b2.x, b2.z)),
-                                 __fadd2_rn(I.s_diag, f2(b1.y, b1.w)));
-    const float sxy = fmaf(fab, I.Rxy + b2.y, I.sxy + b1.z);
-    a.sd_xw = __ffma2_rn(sd, w_xy, a.sd_xw);
-    a.sd_zy = __ffma2_rn(f2(sxy, sxy), w_xy, a.sd_zy);
-    const float2 dvp = __fmul2_rn(dv, pij);
-    const float vijposij = -(dvp.x + dvp.y);
-    const float irhoij = __fdividef(2.f, I.rho + b3.x);
-    if (vijposij < 0.f) {  // Monaghan viscosity for approaching pairs
-      const float cij = 0.5f * (I.c + b3.y);
-      const float hij = 0.5f * (I.h + b2.w);
-      const float muij = hij * vijposij * __fdividef(1.f, fmaf(K.eta2 * hij, hij, rr2));
-      const float npi = fmaf(K.alpha, cij, -K.beta * muij) * muij * irhoij;  // -pi_ij
-      a.vt = __ffma2_rn(f2(npi, npi), w_xy, a.vt);
+  if (I.mech && !f_tool(b0)) {
+    const float dvx = b1.x - I.vx, dvy = b1.y - I.vy;
+    const float ax = __fmul_rn(dvx, volj), ay = __fmul_rn(dvy, volj);
+    a.vdx = fmaf(ax, wx, a.vdx);
+    a.vdy = fmaf(ax, wy, a.vdy);
+    a.vdz = fmaf(ay, wx, a.vdz);
+    a.vdw = fmaf(ay, wy, a.vdw);
+    const float w2 = __fmul_rn(w, w), fab = __fmul_rn(w2, w2);
+    const float sxx = fmaf(fab, I.Rxx + b2.z, I.sxx + b2.x);
+    const float syy = fmaf(fab, I.Ryy + b2.w, I.syy + b2.y);
+    const float sxy = fmaf(fab, I.Rxy + b1.w, I.sxy + b1.z);
+    a.sdx = fmaf(sxx, wx, a.sdx);
+    a.sdw = fmaf(syy, wy, a.sdw);
+    a.sdz = fmaf(sxy, wx, a.sdz);
+    a.sdy = fmaf(sxy, wy, a.sdy);
+    const float nvr = fmaf(dvx, xij, __fmul_rn(dvy, yij));  // -v_ij . x_ij
+    const float irho = __fdividef(1.f, I.rho + b3.x);        // half of 1 / rho_ij
+    if (nvr > 0.f) {  // Monaghan viscosity for approaching pairs: pi_ij / 2
+      const float hh = I.h + fabsf(b0.w);                    // 2 h_ij
+      const float mu2 = __fmul_rn(__fmul_rn(hh, nvr), __fdividef(1.f, fmaf(__fmul_rn(K.eta4, hh), hh, rr2)));
+      const float pi = __fmul_rn(__fmul_rn(fmaf(K.beta4, mu2, __fmul_rn(K.alpha4, I.c + b3.y)), mu2), irho);
+      a.vtx = fmaf(pi, wx, a.vtx);
+      a.vty = fmaf(pi, wy, a.vty);
     }
-    const float xs = w * irhoij;
-    a.xt = __ffma2_rn(f2(xs, xs), dv, a.xt);
+    const float xs = __fmul_rn(w, irho);
+    a.xtx = fmaf(xs, dvx, a.xtx);
+    a.xty = fmaf(xs, dvy, a.xty);
   }
-  // Brookshaw: 2 (m/rho_j)(Ti - Tj)(e_ij . grad W)/r with (e_ij . grad W)/r = der*fac
-  if (I.thermal && rr2 > 1e-16f) a.T_lapl = fmaf(volj * (I.T - b3.w), dwr, a.T_lapl);
+  // Brookshaw: 2 (m/rho_j)(Ti - Tj)(e_ij . grad W)/r with (e_ij . grad W)/r = dwr
+  if (I.thermal && rr2 > 1e-16f) a.T_lapl = fmaf(__fmul_rn(volj, I.T - b3.w), dwr, a.T_lapl);
 }
 
 // Records of the candidates in global memory, read through the read-only path (word k of
-// record j at recf_word(k, j, N)). (A block's candidates staged in shared memory by bulk copies
+// record j among N at recf_word(k, j, N)). (A block's candidates staged in shared memory by bulk copies
 // on one mbarrier measured 25-30 % slower on the ~150k-particle cut: fewer resident warps and
 // the copy's wait before any arithmetic, against loads that L1 already served 84 % of.)
 struct rec_global {
-  const float4 *__restrict__ r;
-  int N;
-  __device__ __forceinline__ float4 p0(int j) const { return __ldg(r + recf_word(0, j, N)); }
+  const float4 *__restrict__ r0;    // word 0
+  const float4 *__restrict__ rest;  // the tiles of words 1..3
+  __device__ __forceinline__ explicit rec_global(const float *recf, int N)
+      : r0(reinterpret_cast<const float4 *>(recf)), rest(r0 + recf_word(1, 0, N)) {}
+  __device__ __forceinline__ float4 p0(int j) const { return __ldg(r0 + j); }
+  __device__ __forceinline__ float4 p3(int j) const { return __ldg(rest + ((size_t)(j >> 5) * 96 + (size_t)(64 + (j & 31)))); }
+  __device__ __forceinline__ void words(int j, float4 &b1, float4 &b2, float4 &b3) const {
+    const float4 *t = rest + ((size_t)(j >> 5) * 96 + (size_t)(j & 31));
+    b1 = __ldg(t); b2 = __ldg(t + 32); b3 = __ldg(t + 64);
+  }
   __device__ __forceinline__ void all(int j, float4 &b0, float4 &b1, float4 &b2, float4 &b3) const {
-    b0 = __ldg(r + recf_word(0, j, N)); b1 = __ldg(r + recf_word(1, j, N));
-    b2 = __ldg(r + recf_word(2, j, N)); b3 = __ldg(r + recf_word(3, j, N));
+    b0 = p0(j);
+    words(j, b1, b2, b3);
   }
 };
 
-// Neighbour list of particle q, built on a step that sorted: the candidates within
-// 2 h_i + skin over the 7x7 cells around its own (the 5x5 window widened by one cell, which
-// covers that radius for h_i up to the cell size), blanked ones left out, non-finite ones
-// kept (their pair terms carry the NaN). Columns in x order and each column's range in array
-// order, so the in-support candidates come in the order of the 5x5 window.
-__device__ __forceinline__ int build_list(const dev_buffers &D, const rec_global &REC, int q,
-                                          const mixed_i &I, const geom &g, int gi, int gj, float dxc,
-                                          float skin) {
+// Neighbour list of particle q (its G lanes, sub = lane), built on a step that sorted: the
+// candidates within 2 h_i + skin over the 7x7 cells around its own (the 5x5 window widened by one
+// cell, which covers that radius for h_i up to the cell size), blanked ones left out, non-finite
+// ones kept (their pair terms carry the NaN). Columns in x order and each column's range in array
+// order. Called by whole warps; `on`: the particle gets a list.
+template <int G>
+__device__ __forceinline__ void build_list(const dev_buffers &D, const rec_global &REC, int q, int sub, bool on,
+                                           const mixed_i &I, const geom &g, int gi, int gj, float dxc, float skin) {
   const float R = 2.f * I.h + skin;
   const float R2 = R * R;
-  const int low_i = gi - 3 < 0 ? 0 : gi - 3;
   const int low_j = gj - 3 < 0 ? 0 : gj - 3;
-  const int high_i = gi + 4 > g.nx ? g.nx : gi + 4;
   const int high_j = gj + 4 > g.ny ? g.ny : gj + 4;
   unsigned *row = D.nlist + (size_t)q * LIST_CAP;
   int cnt = 0;
-  for (int ii = low_i; ii < high_i; ++ii) {
-    const int col = ii * g.ny;
-    const int j0 = __ldg(D.off + col + low_j);
-    const int j1 = __ldg(D.off + col + high_j);
-    const float ox = fmaf((float)(gi - ii), dxc, I.x);
-    const unsigned tag = (unsigned)(gi - ii + 3) << LIST_INDEX_BITS;
-    for (int j = j0; j < j1; ++j) {
-      const float4 b0 = REC.p0(j);
-      const unsigned fjw = (unsigned)__float_as_int(b0.z);
-      const float xij = ox - b0.x;
-      const float yij = fmaf((float)(gj - (int)(fjw >> 8)), dxc, I.y - b0.y);
-      const float rr2 = dist2(xij, yij);
-      if (!(fjw & FLAG_BLANKED) && (!(rr2 >= R2) || (fjw & FLAG_NONFINITE))) {
-        if (cnt < LIST_CAP) row[cnt] = (unsigned)j | tag;
-        ++cnt;
+  for (int c = -3; c <= 3; ++c) {
+    const int ii = gi + c;
+    const bool in = on && ii >= 0 && ii < g.nx;
+    const int j0 = in ? __ldg(D.off + ii * g.ny + low_j) : 0;
+    const int j1 = in ? __ldg(D.off + ii * g.ny + high_j) : 0;
+    const float dcol = (float)-c;
+    const unsigned tag = (unsigned)(3 - c) << LIST_INDEX_BITS;
+    for (int jb = j0; G == 1 ? jb < j1 : __any_sync(0xffffffffu, jb < j1); jb += G) {
+      const int j = jb + sub;
+      bool take = false;
+      if (j < j1) {
+        const float4 b0 = REC.p0(j);
+        take = !f_blanked(b0) && (!(dist2(offset_x(I, b0, dcol, dxc), offset_y(I, b0, dxc)) >= R2) || f_nonfinite(b0));
       }
+      unsigned m = 1u, below = 0u;
+      if (G > 1) {
+        m = (__ballot_sync(0xffffffffu, take) >> (lane_id() & ~(unsigned)(G - 1))) & ((1u << G) - 1u);
+        below = __popc(m & ((1u << sub) - 1u));
+      }
+      if (take && cnt + (int)below < LIST_CAP) row[cnt + below] = (unsigned)j | tag;
+      cnt += G > 1 ? __popc(m) : (take ? 1 : 0);
     }
   }
+  if (!on || sub != 0) return;
   if (cnt > LIST_CAP) {
     atomicOr(&D.st->error_flags, ERR_LIST_OVERFLOW);
     cnt = LIST_CAP;
   }
   D.ncount[q] = cnt;
-  return cnt;
 }
 
 // The neighbour-list invariant by brute force (a diagnostic: all N^2 pairs). k_list_abs puts
@@ -186,10 +211,10 @@ static __global__ void k_list_check(params P, dev_buffers D, const double2 *__re
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.N) return;
   const float4 *__restrict__ r0 = reinterpret_cast<const float4 *>(D.recf);
-  const unsigned fi = (unsigned)__float_as_int(r0[recf_word(0, i, P.N)].z) & 0xffu;
-  if (fi & (FLAG_BLANKED | FLAG_NONFINITE)) return;
-  if ((fi & FLAG_TOOL) && P.thermal_solver != MF_THERMAL_BROOKSHAW) return;  // no pair sums
-  const double h = (double)r0[recf_word(2, i, P.N)].w;
+  const float4 bi = r0[recf_word(0, i, P.N)];
+  if (f_blanked(bi) || f_nonfinite(bi)) return;
+  if (f_tool(bi) && P.thermal_solver != MF_THERMAL_BROOKSHAW) return;  // no pair sums
+  const double h = (double)bi.w;
   const double lim = 4. * h * h * (1. - 1e-5);
   const double2 xi = abs[i];
   const unsigned *row = D.nlist + (size_t)i * LIST_CAP;
@@ -197,8 +222,8 @@ static __global__ void k_list_check(params P, dev_buffers D, const double2 *__re
   unsigned long long pairs = 0, missing = 0;
   for (int j = 0; j < P.N; ++j) {
     if (j == i) continue;
-    const unsigned fj = (unsigned)__float_as_int(r0[recf_word(0, j, P.N)].z);
-    if (fj & (FLAG_BLANKED | FLAG_NONFINITE)) continue;
+    const float4 bj = r0[recf_word(0, j, P.N)];
+    if (f_blanked(bj) || f_nonfinite(bj)) continue;
     const double2 xj = abs[j];
     const double dx = xi.x - xj.x, dy = xi.y - xj.y;
     const double rr2 = dx * dx + dy * dy;
@@ -218,66 +243,40 @@ __device__ __forceinline__ bool mixed_begin(const params &P, const dev_buffers &
                                             mixed_const &K, double &thermal_alpha) {
   if (q >= P.N) return false;
   const float4 *__restrict__ r0 = reinterpret_cast<const float4 *>(D.recf);
-  const float4 a0 = __ldg(r0 + recf_word(0, q, P.N));  // x, y, flags|cy, vx
-  const unsigned fi = (unsigned)__float_as_int(a0.z) & 0xffu;
-  if (fi & FLAG_BLANKED) return false;
-  const bool tool_i = fi & FLAG_TOOL;
+  const float4 a0 = __ldg(r0 + recf_word(0, q, P.N));  // x, y, row, h
+  if (f_blanked(a0)) return false;
+  const bool tool_i = f_tool(a0);
   const bool brookshaw = P.thermal_solver == MF_THERMAL_BROOKSHAW;
   if (!brookshaw && tool_i) return false;
-  const float4 a1 = __ldg(r0 + recf_word(1, q, P.N));  // vy, sxx, sxy, syy
-  const float4 a2 = __ldg(r0 + recf_word(2, q, P.N));  // Rxx, Rxy, Ryy, h
+  const float4 a1 = __ldg(r0 + recf_word(1, q, P.N));  // vx, vy, sxy, Rxy
+  const float4 a2 = __ldg(r0 + recf_word(2, q, P.N));  // sxx, syy, Rxx, Ryy
   const float4 a3 = __ldg(r0 + recf_word(3, q, P.N));  // rho, c, vol, T - T_init
 
-  K.inv_wdeltap = (float)(1. / P.corr.wdeltap);
-  K.alpha = (float)P.corr.alpha;
-  K.beta = (float)P.corr.beta;
+  K.alpha4 = 0.25f * (float)P.corr.alpha;
+  K.beta4 = 0.25f * (float)P.corr.beta;
   const float eta = (float)P.corr.eta;
-  K.eta2 = eta * eta;
+  K.eta4 = 0.25f * eta * eta;
   thermal_alpha = 0.;
   if (brookshaw) thermal_alpha = !tool_i ? P.trml_wp.alpha : (P.thermal_tool_on ? P.trml_tool.alpha : 0.);
 
   I.thermal = thermal_alpha != 0.;
-  I.nonfinite = fi & FLAG_NONFINITE;
+  I.nonfinite = f_nonfinite(a0);
   I.mech = !tool_i;
-  I.x = a0.x; I.y = a0.y; I.nv = f2(-a0.w, -a1.x);
-  I.s_diag = f2(a1.y, a1.w); I.sxy = a1.z;
-  I.r_diag = f2(a2.x, a2.z); I.Rxy = a2.y; I.h = a2.w;
+  I.x = a0.x; I.y = a0.y; I.row = fabsf(a0.z); I.h = fabsf(a0.w);
+  I.vx = a1.x; I.vy = a1.y;
+  I.sxx = a2.x; I.syy = a2.y; I.sxy = a1.z;
+  I.Rxx = a2.z; I.Ryy = a2.w; I.Rxy = a1.w;
   I.rho = a3.x; I.c = a3.y; I.T = I.thermal ? a3.w : 0.f;
-  I.h1 = 1.f / I.h;
-  I.fourh2 = 4.f * I.h * I.h;
-  I.fac = 0.454728408833987f * I.h1 * I.h1;
+  // the spline's constants from the FP64 smoothing length, rounded once: an error of the rounded h
+  // would enter every gradient four times over, all with the same sign
+  const double h = D.B.h[q], h1 = 1. / h, fac = 0.454728408833987 * h1 * h1, w_in = fac * P.inv_wdeltap;
+  I.h1 = (float)h1;
+  I.fourh2 = (float)(4. * h * h);
+  I.w_in = (float)w_in;
+  I.w_out = (float)(0.25 * w_in);
+  I.d_in = (float)(-3. * h1 * h1 * fac);
+  I.d_out = (float)(-0.75 * h1 * fac);
   return true;
-}
-
-// The candidates j0 .. j1 - 1 of one window column (indices into R), in chunks of up to 32: mark
-// the contributing ones, then visit them in order.
-template <class REC>
-__device__ __forceinline__ void mixed_column(const REC &R, int j0, int j1, float ox, int gj, float dxc,
-                                             const mixed_i &I, const mixed_const &K, mixed_acc &acc) {
-  for (int jb = j0; jb < j1; jb += 32) {
-    const int jn = min(32, j1 - jb);
-    unsigned mask = 0u;
-#pragma unroll 4
-    for (int k = 0; k < jn; ++k) {
-      const float4 b0 = R.p0(jb + k);
-      const unsigned fjw = (unsigned)__float_as_int(b0.z);
-      const float xij = ox - b0.x;
-      const float yij = fmaf((float)(gj - (int)(fjw >> 8)), dxc, I.y - b0.y);
-      const float rr2 = dist2(xij, yij);
-      const bool in_support = !(rr2 >= I.fourh2 || rr2 < 1e-8f);
-      const bool take = !(fjw & FLAG_BLANKED) && (in_support || I.nonfinite || (fjw & FLAG_NONFINITE));
-      mask |= (take ? 1u : 0u) << k;
-    }
-    while (mask) {
-      const int k = __ffs(mask) - 1;
-      mask &= mask - 1u;
-      // all four planes at once: one load latency per neighbour
-      float4 b0, b1, b2, b3;
-      R.all(jb + k, b0, b1, b2, b3);
-      const float yij = fmaf((float)(gj - (int)((unsigned)__float_as_int(b0.z) >> 8)), dxc, I.y - b0.y);
-      mixed_interact(I, K, acc, ox - b0.x, yij, b0, b1, b2, b3);
-    }
-  }
 }
 
 // the rates of slot q from its pair sums: Jaumann stress rate, continuity, momentum, advection
@@ -285,12 +284,11 @@ __device__ __forceinline__ void mixed_column(const REC &R, int j0, int j1, float
 __device__ __forceinline__ void mixed_end(const params &P, const dev_buffers &D, int q, int p, const mixed_i &I,
                                           const mixed_acc &acc, double thermal_alpha) {
   const float mass = (float)P.phys.mass;
-  const float m_eps = (float)P.corr.xspheps * mass;
-  const float vdx = acc.vd01.x, vdy = acc.vd01.y, vdz = acc.vd23.x, vdw = acc.vd23.y;
-  const float sdx = mass * acc.sd_xw.x, sdy = mass * acc.sd_zy.y, sdz = mass * acc.sd_zy.x,
-              sdw = mass * acc.sd_xw.y;
-  const float vtx = mass * acc.vt.x, vty = mass * acc.vt.y;
-  const float xtx = m_eps * acc.xt.x, xty = m_eps * acc.xt.y, T_lapl = 2.f * acc.T_lapl;
+  const float m2 = 2.f * mass, m_eps = (float)P.corr.xspheps * m2 * (float)P.corr.wdeltap;
+  const float vdx = acc.vdx, vdy = acc.vdy, vdz = acc.vdz, vdw = acc.vdw;
+  const float sdx = mass * acc.sdx, sdy = mass * acc.sdy, sdz = mass * acc.sdz, sdw = mass * acc.sdw;
+  const float vtx = -m2 * acc.vtx, vty = -m2 * acc.vty;
+  const float xtx = m_eps * acc.xtx, xty = m_eps * acc.xty, T_lapl = 2.f * acc.T_lapl;
   const bool mech_i = I.mech, thermal = I.thermal;
   const float rhoi = I.rho;
 
@@ -316,10 +314,14 @@ __device__ __forceinline__ void mixed_end(const params &P, const dev_buffers &D,
     B.rho_t[q] = -(double)rhoi * (double)(vdx + vdw);
     double2 fc, ft;
     prev_contact_forces(P, D, q, p, fc, ft);
-    const double m = P.phys.mass;
     const double2 vp = B.vel[q];
-    B.vel_t[q] = make_double2((double)(vtx + (sdx + sdy)) + fc.x / m + ft.x / m,
-                              (double)(vty + (sdz + sdw)) + fc.y / m + ft.y / m);
+    double2 vel_t = make_double2((double)(vtx + (sdx + sdy)), (double)(vty + (sdz + sdw)));
+    if (fc.x != 0. || fc.y != 0. || ft.x != 0. || ft.y != 0.) {  // (few particles touch the tool)
+      const double m = P.phys.mass;
+      vel_t.x = vel_t.x + fc.x / m + ft.x / m;
+      vel_t.y = vel_t.y + fc.y / m + ft.y / m;
+    }
+    B.vel_t[q] = vel_t;
     B.pos_t[q] = make_double2((double)xtx + vp.x, (double)xty + vp.y);
   } else {
     B.vel_t[q] = make_double2(vtx, vty);
@@ -328,44 +330,168 @@ __device__ __forceinline__ void mixed_end(const params &P, const dev_buffers &D,
   if (thermal) B.T_t[q] = thermal_alpha * (double)T_lapl;
 }
 
-// LIST: the neighbour-list form (steps with P.verlet)
-template <bool LIST>
-__device__ __forceinline__ void pair_mixed_particle(const params &P, const dev_buffers &D, int q) {
-  mixed_i I;
-  mixed_const K;
-  double thermal_alpha;
-  if (!mixed_begin(P, D, q, I, K, thermal_alpha)) return;
-  const rec_global R{reinterpret_cast<const float4 *>(D.recf), P.N};
-  // the particle's slot at the start of the step (its last contact forces are read there at the
-  // end): loaded now, so that the load's latency passes during the sums; a list step without a
-  // sort keeps the order
-  const bool sorting = !LIST || D.st->sort_now;
-  const int p = sorting ? __ldg(D.perm + q) : q;
+// A particle's contributing neighbours in shared memory, in the order of the window, filled by its
+// G lanes. Its sums have T parts: neighbour number n (counted in that order) belongs to part n mod T,
+// each part is summed in order, and the parts are added up in order. Where T lanes share the
+// particle (G = T) each takes a part; one lane (G = 1, the batched kernels) takes them one after the
+// other and gets the same bits. The neighbours and their order do not depend on whether the window
+// or the particle's neighbour list was searched.
+// An entry is the neighbour's index and the column offset of the pair's cells (i's - j's) + 3.
+template <int G>
+struct mixed_rows {
+  static constexpr int CAP = G == 1 ? 41 : 64 + G;  // entries (rows on distinct banks)
+};
+constexpr int ROW_INDEX_BITS = 29;
+constexpr unsigned ROW_INDEX_MASK = (1u << ROW_INDEX_BITS) - 1u;
+// words of a block's rows, whatever its lanes per particle
+template <int BS>
+struct mixed_shared {
+  static constexpr int WORDS = BS * mixed_rows<1>::CAP;
+};
 
-  const geom g = *D.g;
-  const float dxc = (float)g.dx;
-  const int hashi = D.hash_cur[q];
-  const int gi = hashi / g.ny;
-  const int gj = hashi - gi * g.ny;
+__device__ __forceinline__ void acc_add(mixed_acc &a, const mixed_acc &b) {
+  a.vdx += b.vdx; a.vdy += b.vdy; a.vdz += b.vdz; a.vdw += b.vdw;
+  a.sdx += b.sdx; a.sdy += b.sdy; a.sdz += b.sdz; a.sdw += b.sdw;
+  a.vtx += b.vtx; a.vty += b.vty; a.xtx += b.xtx; a.xty += b.xty;
+  a.T_lapl += b.T_lapl;
+}
+__device__ __forceinline__ void acc_zero(mixed_acc &a) {
+  a.vdx = a.vdy = a.vdz = a.vdw = a.sdx = a.sdy = a.sdz = a.sdw = 0.f;
+  a.vtx = a.vty = a.xtx = a.xty = a.T_lapl = 0.f;
+}
 
-  mixed_acc acc;
-  acc.vd01 = acc.vd23 = acc.sd_xw = acc.sd_zy = acc.vt = acc.xt = f2(0.f, 0.f);
-  acc.T_lapl = 0.f;
+// called by whole warps
+template <int G>
+__device__ __forceinline__ void row_append(unsigned *row, int &cnt, int sub, bool take, unsigned entry) {
+  if (G == 1) {
+    if (take) row[cnt++] = entry;
+    return;
+  }
+  const unsigned m = (__ballot_sync(0xffffffffu, take) >> (lane_id() & ~(unsigned)(G - 1))) & ((1u << G) - 1u);
+  if (take) row[cnt + __popc(m & ((1u << sub) - 1u))] = entry;
+  cnt += __popc(m);
+}
 
-  if (LIST && !I.nonfinite) {
-    // neighbour list: built on a sorting step, then read; each entry passes the same
-    // support test as a window candidate. A particle's row is contiguous: four entries per
-    // 16-byte load; an entry past the count reads the particle's own record (always valid,
-    // so the loads need no guard) and is skipped.
-    const int cnt = sorting ? build_list(D, R, q, I, g, gi, gj, dxc, P.skin) : D.ncount[q];
+// entries first, first + step, ... of a row of cnt
+__device__ __forceinline__ void row_sum(const rec_global &R, const unsigned *row, int first, int step, int cnt,
+                                        const mixed_i &I, const mixed_const &K, float dxc, mixed_acc &acc) {
+  for (int k = first; k < cnt; k += step) {
+    const unsigned e = row[k];
+    float4 b0, b1, b2, b3;
+    R.all((int)(e & ROW_INDEX_MASK), b0, b1, b2, b3);
+    const float dcol = (float)((int)(e >> ROW_INDEX_BITS) - 3);
+    mixed_interact<false>(I, K, acc, offset_x(I, b0, dcol, dxc), offset_y(I, b0, dxc), b0, b1, b2, b3);
+  }
+}
+
+// The row's entries (numbers base, base + 1, ...) into the lane's part of the sums.
+template <int G>
+__device__ __forceinline__ void row_drain(const rec_global &R, const unsigned *row, int &cnt, int &base, int sub,
+                                          const mixed_i &I, const mixed_const &K, float dxc, mixed_acc &acc) {
+  if (G > 1) __syncwarp();
+  row_sum(R, row, (sub - base) & (G - 1), G, cnt, I, K, dxc, acc);
+  base += cnt;
+  cnt = 0;
+  if (G > 1) __syncwarp();
+}
+
+// One lane's T parts, one after the other, added up in acc at the last drain of the particle. Rows
+// that overflow (more than CAP neighbours) keep their unfinished parts in local memory meanwhile.
+template <int T>
+__device__ __forceinline__ void row_drain_parts(const rec_global &R, const unsigned *row, int &cnt, int &base,
+                                                bool last, mixed_acc *part, const mixed_i &I, const mixed_const &K,
+                                                float dxc, mixed_acc &acc) {
+  const bool kept = base != 0;
+#pragma unroll 1
+  for (int r = 0; r < T; ++r) {
+    mixed_acc s;
+    acc_zero(s);
+    if (kept) s = part[r];
+    row_sum(R, row, (r - base) & (T - 1), T, cnt, I, K, dxc, s);
+    if (!last) part[r] = s;
+    else if (r == 0) acc = s;
+    else acc_add(acc, s);
+  }
+  base += cnt;
+  cnt = 0;
+}
+
+// The 5x5 window's pair sums (interactions_gpu.cu:147-345) of a particle's G lanes, in two passes
+// like the FP64 kernel's (pair_fp64_body): the candidates that contribute, by the same FP32 test
+// that the pair term makes, into the row, then the row's entries, so that a warp's lanes run their
+// ~28 pair terms together instead of each column's separately. Called by whole warps; `on`: the
+// particle takes part.
+template <int G, int T>
+__device__ __forceinline__ void mixed_window(const dev_buffers &D, const rec_global &R, int sub, unsigned *row,
+                                             bool on, const mixed_i &I, const mixed_const &K, const geom &g, int gi,
+                                             int gj, float dxc, mixed_acc &acc) {
+  constexpr int STEP = 8, U = STEP / G;
+  static_assert(G == T || G == 1, "a lane per part, or one lane");
+  const int low_j = gj - 2 < 0 ? 0 : gj - 2;
+  const int high_j = gj + 3 > g.ny ? g.ny : gj + 3;
+  int cnt = 0, base = 0;
+  mixed_acc part[G == T ? 1 : T];
+  auto drain = [&](bool last) {
+    if (G == T) row_drain<G>(R, row, cnt, base, sub, I, K, dxc, acc);
+    else row_drain_parts<T>(R, row, cnt, base, last, part, I, K, dxc, acc);
+  };
+  auto bounds = [&](int c, int &j0, int &j1) {  // window column c's particles
+    const int ii = gi - 2 + c;
+    const bool in = on && ii >= 0 && ii < g.nx;
+    j0 = in ? __ldg(D.off + ii * g.ny + low_j) : 0;
+    j1 = in ? __ldg(D.off + ii * g.ny + high_j) : 0;
+  };
+  int n0, n1;
+  bounds(0, n0, n1);
+#pragma unroll 1
+  for (int c = 0; c < 5; ++c) {
+    const int j0 = n0, j1 = n1;
+    if (c < 4) bounds(c + 1, n0, n1);  // the next column's bounds, in flight during this one
+    const float dcol = (float)(2 - c);
+    const unsigned tag = (unsigned)(5 - c) << ROW_INDEX_BITS;
+    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb += STEP) {
+      if (__any_sync(0xffffffffu, cnt > mixed_rows<G>::CAP - STEP)) drain(false);
+      float4 b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        b[u] = R.p0(jb + u * G + sub);  // (past the column's end: not used)
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = jb + u * G + sub;
+        const float rr2 = dist2(offset_x(I, b[u], dcol, dxc), offset_y(I, b[u], dxc));
+        // (false for a blanked particle's NaN row)
+        bool take = rr2 < I.fourh2 && rr2 >= 1e-8f;
+        if (I.nonfinite || f_nonfinite(b[u])) take = !f_blanked(b[u]);
+        row_append<G>(row, cnt, sub, j < j1 && take, (unsigned)j | tag);
+      }
+    }
+  }
+  drain(true);
+}
+
+// A list step's pair sums: the row of the particle's neighbour list in place of the window; each
+// entry passes the same support test as a window candidate. One lane per particle sums as it reads,
+// with a software pipeline: the next entry's four record words are in flight while one entry is
+// summed (past the count, the particle's own record, always a valid address; measured on the
+// ~150k-particle cut: pair kernel 48.1 against 50.1 us at 5 blocks per SM). Several lanes search
+// the list as they search the window. Called by whole warps; `on`: the particle takes part.
+template <int G>
+__device__ __forceinline__ void mixed_list(const dev_buffers &D, const rec_global &R, int q, int sub, unsigned *srow,
+                                           bool on, const mixed_i &I, const mixed_const &K, float dxc, mixed_acc &acc) {
+  const unsigned self = (unsigned)q | (3u << LIST_INDEX_BITS);
+  auto take = [&](const float4 &b0, float xij, float yij) {
+    const float rr2 = dist2(xij, yij);
+    return f_nonfinite(b0) ? !f_blanked(b0) : rr2 < I.fourh2 && rr2 >= 1e-8f;  // (false for a blanked NaN row)
+  };
+  auto xij_of = [&](unsigned e, const float4 &b0) {
+    return offset_x(I, b0, (float)((int)(e >> LIST_INDEX_BITS) - 3), dxc);
+  };
+  const int cnt = on ? D.ncount[q] : 0;
+  if (G == 1) {
+    // a particle's row is contiguous: four entries per 16-byte load
     const uint4 *row = reinterpret_cast<const uint4 *>(D.nlist + (size_t)q * LIST_CAP);
     uint4 e4 = row[0];  // (a row is LIST_CAP entries: the first four are always there)
-    const unsigned self = (unsigned)q | (3u << LIST_INDEX_BITS);
-    // software pipeline: the next entry's four record planes are in flight while one entry is
-    // summed (c0..c3 hold entry k's at the top of its iteration; past the count, the particle's
-    // own record, always a valid address). Measured on the ~150k-particle cut: pair kernel 48.1
-    // against 50.1 us at 5 blocks per SM (96 registers, 4 B of spills); at 4 blocks per SM (108
-    // registers) 54.2 us.
     float4 c0, c1, c2, c3;
     R.all((int)((cnt > 0 ? e4.x : self) & LIST_INDEX_MASK), c0, c1, c2, c3);
     for (int k0 = 0; k0 < cnt; k0 += 4) {
@@ -376,47 +502,110 @@ __device__ __forceinline__ void pair_mixed_particle(const params &P, const dev_b
         const bool live = k0 + u < cnt;
         const unsigned e = live ? ev[u] : self;
         const unsigned en = (k0 + u + 1 < cnt) ? (u < 3 ? ev[u + 1] : e4.x) : self;
-        const float ox = fmaf((float)((int)(e >> LIST_INDEX_BITS) - 3), dxc, I.x);
         const float4 b0 = c0, b1 = c1, b2 = c2, b3 = c3;
         R.all((int)(en & LIST_INDEX_MASK), c0, c1, c2, c3);
-        const unsigned fjw = (unsigned)__float_as_int(b0.z);
-        const float xij = ox - b0.x;
-        const float yij = fmaf((float)(gj - (int)(fjw >> 8)), dxc, I.y - b0.y);
-        const float rr2 = dist2(xij, yij);
-        const bool in_support = !(rr2 >= I.fourh2 || rr2 < 1e-8f);
-        if (live && !(fjw & FLAG_BLANKED) && (in_support || (fjw & FLAG_NONFINITE)))
-          mixed_interact(I, K, acc, xij, yij, b0, b1, b2, b3);
+        const float xij = xij_of(e, b0), yij = offset_y(I, b0, dxc);
+        if (live && take(b0, xij, yij)) mixed_interact<true>(I, K, acc, xij, yij, b0, b1, b2, b3);
       }
     }
-  } else {  // the 5x5 window (interactions_gpu.cu:147-345)
-    const int low_i = gi - 2 < 0 ? 0 : gi - 2;
-    const int low_j = gj - 2 < 0 ? 0 : gj - 2;
-    const int high_i = gi + 3 > g.nx ? g.nx : gi + 3;
-    const int high_j = gj + 3 > g.ny ? g.ny : gj + 3;
-    for (int ii = low_i; ii < high_i; ++ii) {
-      const int col = ii * g.ny;
-      const int j0 = __ldg(D.off + col + low_j);
-      const int j1 = __ldg(D.off + col + high_j);
-      mixed_column(R, j0, j1, fmaf((float)(gi - ii), dxc, I.x), gj, dxc, I, K, acc);
+    return;
+  }
+  constexpr int U = 8 / G;
+  static_assert(G == 1 || LIST_CAP <= mixed_rows<G>::CAP, "a whole list fits a row");
+  const unsigned *row = D.nlist + (size_t)q * LIST_CAP;
+  int n = 0, base = 0;
+  for (int k0 = 0; __any_sync(0xffffffffu, k0 < cnt); k0 += 8) {
+    unsigned e[U];
+    float4 b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = k0 + u * G + sub < cnt ? row[k0 + u * G + sub] : self;
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = R.p0((int)(e[u] & LIST_INDEX_MASK));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = take(b[u], xij_of(e[u], b[u]), offset_y(I, b[u], dxc));
+      row_append<G>(srow, n, sub, k0 + u * G + sub < cnt && in,
+                    (e[u] & LIST_INDEX_MASK) | (e[u] >> LIST_INDEX_BITS << ROW_INDEX_BITS));
     }
   }
-  mixed_end(P, D, q, p, I, acc, thermal_alpha);
+  row_drain<G>(R, srow, n, base, sub, I, K, dxc, acc);
 }
 
-// the mixed pair sums of block bk.x's particles
-template <bool LIST>
-__device__ __forceinline__ void pair_mixed_body(const params &P, const dev_buffers &D, blk bk) {
-  pair_mixed_particle<LIST>(P, D, bk.x * blockDim.x + threadIdx.x);
+// The mixed pair sums, in T parts, of the particles of block bk.x (BS threads, G lanes per particle;
+// s_list: mixed_shared<BS>::WORDS words). LIST: the neighbour-list form (steps with P.verlet): a step that
+// sorts sums over the window, exactly as the form without lists, and builds the lists; the steps
+// that keep the order sum over the lists (a particle with a non-finite record over the window).
+template <int BS, int G, int T, bool LIST>
+__device__ __forceinline__ void pair_mixed_body(const params &P, const dev_buffers &D, blk bk, unsigned *s_list) {
+  const int sub = (int)threadIdx.x & (G - 1);
+  const int q = bk.x * (BS / G) + (int)threadIdx.x / G;
+  const int qc = q < P.N ? q : P.N - 1;
+  unsigned *const row = s_list + (int)threadIdx.x / G * mixed_rows<G>::CAP;
+  mixed_i I;
+  mixed_const K;
+  double thermal_alpha;
+  const bool act = mixed_begin(P, D, qc, I, K, thermal_alpha) && q < P.N;
+  if (!__any_sync(0xffffffffu, act)) return;
+  const rec_global R(D.recf, P.N);
+  // the particle's slot at the start of the step (its last contact forces are read there at the
+  // end): loaded now, so that the load's latency passes during the sums; a list step without a
+  // sort keeps the order
+  const bool sorting = !LIST || D.st->sort_now;
+  const int p = sorting ? __ldg(D.perm + qc) : qc;
+
+  const geom g = *D.g;
+  const float dxc = (float)g.dx;
+  const int gi = D.col[qc];
+  const int gj = (int)I.row - 1;
+
+  mixed_acc acc;
+  acc_zero(acc);
+
+  const bool window = act && (sorting || I.nonfinite);
+  if (LIST && !sorting) {
+    mixed_list<G>(D, R, qc, sub, row, act && !window, I, K, dxc, acc);
+    __syncwarp();
+  }
+  if (!LIST || __any_sync(0xffffffffu, window))
+    mixed_window<G, T>(D, R, sub, row, window, I, K, g, gi, gj, dxc, acc);
+  if (LIST && sorting) build_list<G>(D, R, qc, sub, act && !I.nonfinite, I, g, gi, gj, dxc, P.skin);
+  if (G > 1) {  // the lanes' parts, added up in order by the particle's first lane
+    const mixed_acc own = acc;
+#pragma unroll
+    for (int r = 1; r < G; ++r) {
+      mixed_acc o;
+      o.vdx = __shfl_down_sync(0xffffffffu, own.vdx, r); o.vdy = __shfl_down_sync(0xffffffffu, own.vdy, r);
+      o.vdz = __shfl_down_sync(0xffffffffu, own.vdz, r); o.vdw = __shfl_down_sync(0xffffffffu, own.vdw, r);
+      o.sdx = __shfl_down_sync(0xffffffffu, own.sdx, r); o.sdy = __shfl_down_sync(0xffffffffu, own.sdy, r);
+      o.sdz = __shfl_down_sync(0xffffffffu, own.sdz, r); o.sdw = __shfl_down_sync(0xffffffffu, own.sdw, r);
+      o.vtx = __shfl_down_sync(0xffffffffu, own.vtx, r); o.vty = __shfl_down_sync(0xffffffffu, own.vty, r);
+      o.xtx = __shfl_down_sync(0xffffffffu, own.xtx, r); o.xty = __shfl_down_sync(0xffffffffu, own.xty, r);
+      o.T_lapl = __shfl_down_sync(0xffffffffu, own.T_lapl, r);
+      acc_add(acc, o);
+    }
+  }
+  if (act && sub == 0) mixed_end(P, D, q, p, I, acc, thermal_alpha);
 }
 
-// blocks per SM: the window kernel at 6 (80 registers, no spills); the list kernel at 5 (96
-// registers with its software pipeline, 4 B of spills; before the pipeline, at 6 it spilled a
-// little and ran ~1.5 us slower than at 5, at 9 with 56 registers 13 us slower)
-template <bool LIST>
+// Parts of a particle's sums, and lanes per particle of the single-system kernels: as many as let
+// every particle's lanes be resident at once (24 warps per SM on 148 SMs: 28,416 particles at 4;
+// 20 warps of the list form: 47,360 at 2), then one; see pair64_lanes. Pair stage in us (launch
+// included) sorted every step / on lists, at 1 lane: 7,096 particles 19.5 / 21.5; 23,416 23.5 / 22.1;
+// 45,052 27.6 / 24.2; 70,316 31.7 / 27.7; 176,695 55 / 49; at 2: 17.4 / 17.3; 19.5 / 17.4; 23.6 /
+// 21.4; 31.7 / 31.6; 58 / 60; at 4: 15.4 / 13.3; 17.4 / 14.3; 25.6 / 21.5; 35.8 / 29.7; 71 / 67.
+// (Before, one thread per particle: 22.0 on lists at 6,149, 32.8 sorted at 45,052, 52 on lists at 176,695.)
+// A batch of many small systems fills the GPU anyway and runs them at one lane, in as many parts
+// (24 systems of 2.8k to 38k particles: 196 us a step at one lane, 209 at two, 253 at four).
+__host__ __device__ constexpr int mixed_parts(int N) { return N <= 28416 ? 4 : N <= 47360 ? 2 : 1; }
+
+// blocks per SM: the window form at 6 (80 registers, no spills), the list form at 5 (96 registers,
+// its software pipeline; at 4 with 113 registers 54 against 48 us)
+template <int G, bool LIST>
 static __global__ void __launch_bounds__(PAIR_BLOCK, LIST ? 5 : 6) k_pair_mixed(params P, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
-  pair_mixed_body<LIST>(P, D, grid_blk());
+  __shared__ unsigned s_list[PAIR_BLOCK / G * mixed_rows<G>::CAP];
+  pair_mixed_body<PAIR_BLOCK, G, G, LIST>(P, D, grid_blk(), s_list);
 }
 
 // PSE heat Laplacian (interactions_gpu.cu:88-144, kernels.cuh:72-89) in FP32 for the mixed
@@ -426,23 +615,22 @@ static __global__ void __launch_bounds__(PAIR_BLOCK, LIST ? 5 : 6) k_pair_mixed(
 __device__ __forceinline__ void pse_mixed_body(const params &P, const dev_buffers &D, blk bk) {
   const int q = bk.x * blockDim.x + threadIdx.x;
   if (q >= P.N) return;
-  const float4 *__restrict__ r = reinterpret_cast<const float4 *>(D.recf);
-  const float4 a0 = __ldg(r + recf_word(0, q, P.N));  // x, y, flags|cy, vx
-  const unsigned fi = (unsigned)__float_as_int(a0.z) & 0xffu;
-  if (fi & FLAG_BLANKED) return;
-  const float hi = __ldg(r + recf_word(2, q, P.N)).w;
-  const float Ti = __ldg(r + recf_word(3, q, P.N)).w;
+  const rec_global R(D.recf, P.N);
+  const float4 a0 = R.p0(q);  // x, y, row, h
+  if (f_blanked(a0)) return;
+  const float hi = fabsf(a0.w);
+  const float Ti = R.p3(q).w;
   const long long tex_elems = ((long long)sizeof(int) * P.N) / 8;
-  const bool tool_i = q < tex_elems ? (fi & FLAG_TOOL) != 0 : false;
+  const bool tool_i = q < tex_elems ? f_tool(a0) : false;
   const double alpha = tool_i ? P.trml_tool.alpha : P.trml_wp.alpha;
   const float h2 = hi * hi;
   const float inv_h2 = 1.f / h2;
   const float coef = (float)(4. / 3.14159265358979323846) / (h2 * h2);
   const geom g = *D.g;
   const float dxc = (float)g.dx;
-  const int hashi = D.hash_cur[q];
-  const int gi = hashi / g.ny;
-  const int gj = hashi - gi * g.ny;
+  const float row = fabsf(a0.z);
+  const int gi = D.col[q];
+  const int gj = (int)row - 1;
   const int low_i = gi - 2 < 0 ? 0 : gi - 2;
   const int low_j = gj - 2 < 0 ? 0 : gj - 2;
   const int high_i = gi + 3 > g.nx ? g.nx : gi + 3;
@@ -454,10 +642,12 @@ __device__ __forceinline__ void pse_mixed_body(const params &P, const dev_buffer
     const float ox = (float)(gi - ii) * dxc + a0.x;
 #pragma unroll 4
     for (int j = j0; j < j1; ++j) {
-      const float4 b0 = __ldg(r + recf_word(0, j, P.N));
-      const float4 b3 = __ldg(r + recf_word(3, j, P.N));  // rho, c, vol, T - T_init
+      const float4 b0 = R.p0(j);
+      const float4 b3 = R.p3(j);  // rho, c, vol, T - T_init
       const float xij = ox - b0.x;
-      const float yij = fmaf((float)(gj - (int)((unsigned)__float_as_int(b0.z) >> 8)), dxc, a0.y - b0.y);
+      float jrow = fabsf(b0.z);
+      if (f_blanked(b0)) jrow = (float)(D.hash_cur[j] - ii * g.ny + 1);
+      const float yij = fmaf(row - jrow, dxc, a0.y - b0.y);
       const float w2 = coef * __expf(-(xij * xij + yij * yij) * inv_h2);
       T_ti += (b3.w - Ti) * w2 * b3.z;
     }

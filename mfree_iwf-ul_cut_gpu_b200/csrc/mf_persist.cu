@@ -114,6 +114,7 @@ __device__ __forceinline__ void persist_phase(const batch_map &m, int nvb, batch
 
 __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args A) {
   __shared__ batch_entry s;
+  __shared__ unsigned s_list[mixed_shared<PERSIST_BLOCK>::WORDS];
   for (int st = 0; st < A.K; ++st) {
     const batch_entry *ent = A.e + (size_t)(st & 1) * A.n;
     const batch_map m_scan{ent, A.first, A.n}, m_256{ent, A.first + (A.n + 1), A.n},
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args 
     if (!persist_sync(A)) return;
     persist_phase(m_256, A.grid[1], s, [&](blk b) { reorder_body<true, true>(s.P, s.D, b); });
     if (!persist_sync(A)) return;
-    persist_phase(m_pair, A.grid[2], s, [&](blk b) { pair_mixed_body<false>(s.P, s.D, b); });
+    persist_phase(m_pair, A.grid[2], s, [&](blk b) { pair_mixed_system<PERSIST_BLOCK>(s.P, s.D, b, s_list); });
     if (!persist_sync(A)) return;
     if (A.pse) {
       persist_phase(m_pair, A.grid[2], s, [&](blk b) { pse_mixed_body(s.P, s.D, b); });

@@ -372,8 +372,7 @@ __global__ void __launch_bounds__(T_PAIR_BLOCK, 5) k_t_pair(params P, dev_buffer
       float4 b[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int j = jb + u * G + sub;
-        b[u] = __ldg(cand + (j < j1 ? j : qc));
+        b[u] = __ldg(cand + (jb + u * G + sub));  // (past the column's end: not used)
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -807,7 +806,7 @@ int run_mean_force(const params &P_in, const dev_buffers &C, const state_set &no
     m.get(T.sa.flags, (size_t)N);
     m.get(T.sb.flags, (size_t)N);
     m.get(T.fl, (size_t)N);
-    m.get(T.cand, (size_t)N);
+    m.get(T.cand, (size_t)N + CAND_PAD);
     m.get(T.blk, 4 * (size_t)nf * nd);
     m.get(T.n, 2 * (size_t)N * nd);
     m.get(T.pp, (size_t)N * nd);
