@@ -745,6 +745,9 @@ struct arena {
   }
 };
 
+// each kernel may be scheduled while the previous one drains: launched one by one, not from a graph, the
+// steps lose more to the gaps than the early start's uneven spread costs (1,045 against 1,143 us for
+// 16 steps of 6,149 particles with the pair and finish kernels in turn)
 template <typename... KArgs, typename... Args>
 cudaError_t launch(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, int block, Args... args) {
   cudaLaunchConfig_t cfg = {};
