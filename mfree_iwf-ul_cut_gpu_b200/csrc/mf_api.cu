@@ -181,6 +181,7 @@ int alloc_particles(mf_ctx *ctx, int N) {
   TRY(dalloc(ctx, L, &D.rec, rec_doubles(N) + ((size_t)N + CAND_PAD) * 2));  // pair records, candidate records
   TRY(dalloc(ctx, L, &D.recf, recf_floats(N)));
   TRY(dalloc(ctx, L, &D.col, N));
+  TRY(dalloc(ctx, L, &D.heat, (size_t)N + CAND_PAD));
   TRY(dalloc(ctx, L, &D.S_der, N));
   TRY(dalloc(ctx, L, &D.v_der, N));
   TRY(dalloc(ctx, L, &D.hash_cur, N));
@@ -339,6 +340,23 @@ int launch_pair_mixed(mf_ctx *ctx) {
   }
 }
 
+int launch_pse(mf_ctx *ctx) {
+  const int lanes = pair64_lanes(ctx->N), per = PAIR_BLOCK / lanes, nb = (ctx->N + per - 1) / per;
+  switch (lanes) {
+    case 4: return launch(ctx, IN_TURN, k_pse<4>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    case 2: return launch(ctx, IN_TURN, k_pse<2>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    default: return launch(ctx, IN_TURN, k_pse<1>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+  }
+}
+int launch_pse_mixed(mf_ctx *ctx) {
+  const int lanes = mixed_parts(ctx->N), per = PAIR_BLOCK / lanes, nb = (ctx->N + per - 1) / per;
+  switch (lanes) {
+    case 4: return launch(ctx, IN_TURN, k_pse_mixed<4>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    case 2: return launch(ctx, IN_TURN, k_pse_mixed<2>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+    default: return launch(ctx, IN_TURN, k_pse_mixed<1>, nb, PAIR_BLOCK, ctx->P, ctx->D);
+  }
+}
+
 int launch_stage(mf_ctx *ctx, int stage) {
   static const char *const names[4] = {"mf stage 0: cell list", "mf stage 1: predictor",
                                        "mf stage 2: pair sums", "mf stage 3: finish + return map"};
@@ -361,8 +379,7 @@ int launch_stage(mf_ctx *ctx, int stage) {
       if (mixed) TRY(ctx->P.verlet ? launch_pair_mixed<true>(ctx) : launch_pair_mixed<false>(ctx));
       else TRY(launch_pair_fp64(ctx));
       if (ctx->P.thermal_solver == MF_THERMAL_PSE && ctx->P.thermal_wp) {
-        if (mixed) TRY(launch(ctx, IN_TURN, k_pse_mixed, npb, PAIR_BLOCK, ctx->P, ctx->D));
-        else TRY(launch(ctx, IN_TURN, k_pse, npb, PAIR_BLOCK, ctx->P, ctx->D));
+        TRY(mixed ? launch_pse_mixed(ctx) : launch_pse(ctx));
       }
       break;
     case 3:

@@ -125,7 +125,20 @@ static __global__ void __launch_bounds__(BS) kb_pse(batch_map M) {
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  pse_body(s.P, s.D, b);
+  switch (pair64_lanes(s.P.N)) {
+    case 4: pse_body<BS, 4>(s.P, s.D, b); break;
+    case 2: pse_body<BS, 2>(s.P, s.D, b); break;
+    default: pse_body<BS, 1>(s.P, s.D, b); break;
+  }
+}
+
+template <int BS>
+__device__ __forceinline__ void pse_mixed_system(const params &P, const dev_buffers &D, blk b) {
+  switch (mixed_parts(P.N)) {
+    case 4: pse_mixed_body<BS, 4>(P, D, b); break;
+    case 2: pse_mixed_body<BS, 2>(P, D, b); break;
+    default: pse_mixed_body<BS, 1>(P, D, b); break;
+  }
 }
 
 template <int BS>
@@ -134,7 +147,7 @@ static __global__ void __launch_bounds__(BS) kb_pse_mixed(batch_map M) {
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  pse_mixed_body(s.P, s.D, b);
+  pse_mixed_system<BS>(s.P, s.D, b);
 }
 
 static __global__ void __launch_bounds__(FINISH_BLOCK, 2) kb_finish(batch_map M) {

@@ -153,14 +153,6 @@ __device__ __forceinline__ void cubic_spline_fp64(double xij, double yij, double
   dwr = der * fac;
 }
 
-// PSE Laplacian kernel (kernels.cuh:72-89)
-__device__ __forceinline__ double lapl_pse_fp64(double xij, double yij, double hi) {
-  double xx = sqrt(xij * xij + yij * yij);
-  double h2 = hi * hi;
-  double h4 = h2 * h2;
-  return +4. / (h4 * 3.14159265358979323846) * exp(-xx * xx / (h2));
-}
-
 // ---------------------------------------------------------------------------------------
 // artificial stress (actions_gpu.cu:35-39, 53-97)
 __device__ __forceinline__ void artificial_stress(double rhoi, double pi, double Sx, double Sy, double Sz,

@@ -133,7 +133,6 @@ struct rec_global {
   __device__ __forceinline__ explicit rec_global(const float *recf, int N)
       : r0(reinterpret_cast<const float4 *>(recf)), rest(r0 + recf_word(1, 0, N)) {}
   __device__ __forceinline__ float4 p0(int j) const { return __ldg(r0 + j); }
-  __device__ __forceinline__ float4 p3(int j) const { return __ldg(rest + ((size_t)(j >> 5) * 96 + (size_t)(64 + (j & 31)))); }
   __device__ __forceinline__ void words(int j, float4 &b1, float4 &b2, float4 &b3) const {
     const float4 *t = rest + ((size_t)(j >> 5) * 96 + (size_t)(j & 31));
     b1 = __ldg(t); b2 = __ldg(t + 32); b3 = __ldg(t + 64);
@@ -611,54 +610,85 @@ static __global__ void __launch_bounds__(PAIR_BLOCK, LIST ? 5 : 6) k_pair_mixed(
 // PSE heat Laplacian (interactions_gpu.cu:88-144, kernels.cuh:72-89) in FP32 for the mixed
 // form, on the FP32 records: the same window (every particle of the 5x5 cells, blanked ones
 // included, no support cut-off) and the same alpha through the half-length texture binding;
-// exp from the hardware approximation, temperatures relative to the initial temperature.
+// the Gaussian from the hardware's 2^x, its exponent's factor rounded once from the FP64 smoothing
+// length, temperatures relative to the initial temperature. G lanes per particle as in pse_body.
+// It is bound by instructions (56 candidates of a particle), so a round of 8 candidates is read at
+// constant offsets from one address (past the column's end what is read is not used), and a blanked
+// candidate, whose record holds no row, is noticed by the NaN it leaves and the round done again.
+// Measured at 577,555 particles: 54.9 us before (41 instructions a candidate), 48.3 so.
+template <int BS, int G>
 __device__ __forceinline__ void pse_mixed_body(const params &P, const dev_buffers &D, blk bk) {
-  const int q = bk.x * blockDim.x + threadIdx.x;
-  if (q >= P.N) return;
+  constexpr int U = 8 / G, GROUPS = BS / G;
+  const int sub = (int)threadIdx.x & (G - 1);
   const rec_global R(D.recf, P.N);
-  const float4 a0 = R.p0(q);  // x, y, row, h
-  if (f_blanked(a0)) return;
-  const float hi = fabsf(a0.w);
-  const float Ti = R.p3(q).w;
-  const long long tex_elems = ((long long)sizeof(int) * P.N) / 8;
-  const bool tool_i = q < tex_elems ? f_tool(a0) : false;
-  const double alpha = tool_i ? P.trml_tool.alpha : P.trml_wp.alpha;
-  const float h2 = hi * hi;
-  const float inv_h2 = 1.f / h2;
-  const float coef = (float)(4. / 3.14159265358979323846) / (h2 * h2);
+  const float2 *__restrict__ heat = D.heat;
+  const int N = P.N;
   const geom g = *D.g;
   const float dxc = (float)g.dx;
-  const float row = fabsf(a0.z);
-  const int gi = D.col[q];
-  const int gj = (int)row - 1;
-  const int low_i = gi - 2 < 0 ? 0 : gi - 2;
-  const int low_j = gj - 2 < 0 ? 0 : gj - 2;
-  const int high_i = gi + 3 > g.nx ? g.nx : gi + 3;
-  const int high_j = gj + 3 > g.ny ? g.ny : gj + 3;
-  float T_ti = 0.f;
-  for (int ii = low_i; ii < high_i; ++ii) {
-    const int j0 = __ldg(D.off + ii * g.ny + low_j);
-    const int j1 = __ldg(D.off + ii * g.ny + high_j);
-    const float ox = (float)(gi - ii) * dxc + a0.x;
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j) {
-      const float4 b0 = R.p0(j);
-      const float4 b3 = R.p3(j);  // rho, c, vol, T - T_init
-      const float xij = ox - b0.x;
-      float jrow = fabsf(b0.z);
-      if (f_blanked(b0)) jrow = (float)(D.hash_cur[j] - ii * g.ny + 1);
-      const float yij = fmaf(row - jrow, dxc, a0.y - b0.y);
-      const float w2 = coef * __expf(-(xij * xij + yij * yij) * inv_h2);
-      T_ti += (b3.w - Ti) * w2 * b3.z;
+  const long long tex_elems = ((long long)sizeof(int) * P.N) / 8;
+  for (int q0 = bk.x * GROUPS; q0 < N; q0 += bk.n * GROUPS) {
+    const int q = q0 + (int)threadIdx.x / G, qc = min(q, N - 1);
+    const float4 a0 = R.p0(qc);  // x, y, row, h
+    const float Ti = __ldg(heat + qc).y;
+    const double h = D.B.h[qc], h2 = h * h;
+    const float k2 = (float)(-1.4426950408889634 / h2);  // exp(-r^2 / h^2) = 2^(k2 r^2)
+    const bool act = q < N && !f_blanked(a0);
+    const float row = fabsf(a0.z);
+    const int gi = D.col[qc], gj = (int)row - 1;
+    const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
+    float sum = 0.f;
+    auto term = [&](const float4 &b0, float jrow, const float2 &b, float dcol) {
+      const float xij = fmaf(dcol, dxc, a0.x - b0.x), yij = fmaf(row - jrow, dxc, a0.y - b0.y);
+      float w;
+      asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmul_rn(dist2(xij, yij), k2)));
+      return make_float2(__fmul_rn(b.y - Ti, b.x), w);
+    };
+    if (act) {
+      for (int ii = max(gi - 2, 0); ii < min(gi + 3, g.nx); ++ii) {
+        const int j0 = __ldg(D.off + ii * g.ny + low_j);
+        const int j1 = __ldg(D.off + ii * g.ny + high_j);
+        const float dcol = (float)(gi - ii);
+        for (int jb = j0 + sub; jb < j1; jb += 8) {
+          float4 b0[U];
+          float2 b[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            b0[u] = R.p0(jb + u * G);
+            b[u] = __ldg(heat + (jb + u * G));
+          }
+          const float before = sum;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const float2 t = term(b0[u], fabsf(b0[u].z), b[u], dcol);
+            if (jb + u * G < j1) sum = fmaf(t.x, t.y, sum);
+          }
+          if (sum != sum) {  // a blanked candidate (or a NaN): its row from its cell
+            sum = before;
+            for (int j = jb; j < min(jb + 8, j1); j += G) {
+              const float4 c0 = R.p0(j);
+              const float jrow = f_blanked(c0) ? (float)(D.hash_cur[j] - ii * g.ny + 1) : fabsf(c0.z);
+              const float2 t = term(c0, jrow, __ldg(heat + j), dcol);
+              sum = fmaf(t.x, t.y, sum);
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (act && sub == 0) {
+      const bool tool_i = q < tex_elems ? f_tool(a0) : false;
+      const double alpha = tool_i ? P.trml_tool.alpha : P.trml_wp.alpha;
+      D.B.T_t[q] = alpha * (4. / 3.14159265358979323846 / (h2 * h2) * (double)sum);
     }
   }
-  D.B.T_t[q] = alpha * (double)T_ti;
 }
 
+template <int G>
 static __global__ void __launch_bounds__(PAIR_BLOCK) k_pse_mixed(params P, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
-  pse_mixed_body(P, D, grid_blk());
+  pse_mixed_body<PAIR_BLOCK, G>(P, D, grid_blk());
 }
 
 }  // namespace mf

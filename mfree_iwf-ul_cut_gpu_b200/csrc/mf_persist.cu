@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args 
     persist_phase(m_pair, A.grid[2], s, [&](blk b) { pair_mixed_system<PERSIST_BLOCK>(s.P, s.D, b, s_list); });
     if (!persist_sync(A)) return;
     if (A.pse) {
-      persist_phase(m_pair, A.grid[2], s, [&](blk b) { pse_mixed_body(s.P, s.D, b); });
+      persist_phase(m_pair, A.grid[2], s, [&](blk b) { pse_mixed_system<PERSIST_BLOCK>(s.P, s.D, b); });
       if (!persist_sync(A)) return;
     }
     persist_phase(m_256, A.grid[1], s, [&](blk b) { finish_flat_body<true, false>(s.P, s.D, s.scan_tiles, b); });
