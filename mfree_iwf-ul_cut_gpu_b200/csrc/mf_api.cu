@@ -193,13 +193,9 @@ int alloc_particles(mf_ctx *ctx, int N) {
   TRY(dalloc(ctx, L, &D.ncount, N));
   TRY(dalloc(ctx, L, &D.pos_build, N));
   ctx->bbox_blocks = std::min((N + BLOCK - 1) / BLOCK, ctx->sm_count * 4);
-  // per-chunk force partials of the finish kernel and their group sums (or per-block partials of
-  // the bbox pass), the force sum's group tickets
+  // per-block force partials of the finish kernel (or of the bbox and tool wear passes)
   const int finish_chunks = (N + FINISH_BLOCK - 1) / FINISH_BLOCK;
-  const int force_groups = (finish_chunks + FORCE_GROUP - 1) / FORCE_GROUP;
-  TRY(dalloc(ctx, L, &D.partials,
-             (size_t)std::max(std::max(finish_chunks + force_groups, ctx->bbox_blocks), 1) * 8));
-  TRY(dalloc(ctx, L, &D.gticket, (size_t)std::max(force_groups, 1)));
+  TRY(dalloc(ctx, L, &D.partials, (size_t)std::max(std::max(finish_chunks, ctx->bbox_blocks), 1) * 8));
   TRY(invalidate_counts(ctx));
   ctx->N = N;
   return MF_OK;
@@ -363,7 +359,6 @@ int launch_stage(mf_ctx *ctx, int stage) {
   nvtx_range range(stage >= 0 && stage < 4 ? names[stage] : "mf stage");
   const int N = ctx->N;
   const int nb = (N + BLOCK - 1) / BLOCK;
-  const int npb = (N + PAIR_BLOCK - 1) / PAIR_BLOCK;
   bind_sets(ctx);
   set_list_mode(ctx);
   const bool mixed = ctx->P.precision == MF_PRECISION_MIXED;
@@ -388,29 +383,31 @@ int launch_stage(mf_ctx *ctx, int stage) {
         const bool hash = fused_step(ctx);
         if (ctx->P.h_contact > 0.) {  // with contact conductance
           if (ctx->P.fuse && hash)
-            TRY(launch(ctx, IN_TURN, k_finish_flat<true, true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<true, true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
           else if (ctx->P.fuse)
-            TRY(launch(ctx, IN_TURN, k_finish_flat<false, true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<false, true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
           else if (hash)
-            TRY(launch(ctx, IN_TURN, k_finish_flat<true, false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<true, false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
           else
-            TRY(launch(ctx, IN_TURN, k_finish_flat<false, false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<false, false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
         } else if (ctx->P.fuse) {  // the next step's predictor runs here too
           if (hash)
-            TRY(launch(ctx, IN_TURN, k_finish_flat<true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<true, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
           else
-            TRY(launch(ctx, IN_TURN, k_finish_flat<false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+            TRY(launch(ctx, IN_TURN, k_finish_flat<false, true>, fb, FINISH_BLOCK, ctx->P, ctx->D));
         } else if (hash) {
-          TRY(launch(ctx, IN_TURN, k_finish_flat<true, false>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+          TRY(launch(ctx, IN_TURN, k_finish_flat<true, false>, fb, FINISH_BLOCK, ctx->P, ctx->D));
         } else {
-          TRY(launch(ctx, IN_TURN, k_finish_flat<false, false>, fb, FINISH_BLOCK, ctx->P, ctx->D, ctx->scan_tiles));
+          TRY(launch(ctx, IN_TURN, k_finish_flat<false, false>, fb, FINISH_BLOCK, ctx->P, ctx->D));
         }
       }
       if (ctx->P.plastic) {
         if (ctx->P.jc_model == MF_JC_TANH)
-          TRY(launch(ctx, EARLY, k_plastic<false>, ctx->sm_count * PLASTIC_BLOCKS_PER_SM, BLOCK, ctx->P, ctx->D));
+          TRY(launch(ctx, EARLY, k_plastic<false>, ctx->sm_count * PLASTIC_BLOCKS_PER_SM + 1, BLOCK, ctx->P, ctx->D));
         else
-          TRY(launch(ctx, EARLY, k_plastic<true>, ctx->sm_count * PLASTIC_BLOCKS_PER_SM, BLOCK, ctx->P, ctx->D));
+          TRY(launch(ctx, EARLY, k_plastic<true>, ctx->sm_count * PLASTIC_BLOCKS_PER_SM + 1, BLOCK, ctx->P, ctx->D));
+      } else {
+        TRY(launch(ctx, EARLY, k_close, 1, BLOCK, ctx->P, ctx->D));
       }
       break;
     default:
@@ -753,6 +750,23 @@ int mf_get_field(mf_ctx *ctx, int field, void *host) {
   return MF_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// a host write of the contact forces or normals: every particle is marked as holding some
+__global__ void k_mark_touch(int N, unsigned *flags) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) flags[i] |= FLAG_TOUCH;
+}
+bool touch_field(int f) { return f == MF_FIELD_FC || f == MF_FIELD_FT || f == MF_FIELD_N; }
+cudaError_t mark_touch(mf_ctx *ctx, cudaStream_t st) {
+  k_mark_touch<<<(ctx->N + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(ctx->N, ctx->set[view_set(ctx)].flags);
+  return cudaGetLastError();
+}
+}  // namespace
+
+extern "C" {
+
 int mf_set_field(mf_ctx *ctx, int field, const void *host) {
   if (!ctx || !host || field < 0 || field >= MF_NUM_FIELDS) return MF_ERR_INVALID;
   if (!ctx->has_particles) return MF_ERR_STATE;
@@ -777,6 +791,7 @@ int mf_set_field(mf_ctx *ctx, int field, const void *host) {
   if (!dst) return MF_ERR_INVALID;
   size_t bytes = N * d.width * (d.is_int ? sizeof(int) : sizeof(double));
   CK(cudaMemcpy(dst, host, bytes, cudaMemcpyHostToDevice));
+  if (touch_field(field)) CK(mark_touch(ctx, ctx->stream));
   return MF_OK;
 }
 
@@ -793,6 +808,7 @@ int mf_grid_create_locked(mf_ctx *ctx, int kind, double bbmin_x, double bbmin_y,
   G.bbmax_y = bbmax_y + 1e-6;
   double kernel_width = 2.;
   G.dx = h * kernel_width / 2.;
+  G.inv_dx = 1. / G.dx;
   double lx = G.bbmax_x - G.bbmin_x, ly = G.bbmax_y - G.bbmin_y;
   double fnx = std::ceil(lx / G.dx), fny = std::ceil(ly / G.dx);
   if (!(fnx >= 1. && fny >= 1.) || fnx * fny > 2.0e9) return MF_ERR_RANGE;
@@ -816,7 +832,7 @@ int mf_grid_create_adaptive(mf_ctx *ctx, int kind, int max_cell) {
   TRY(set_device(ctx));
   CK(cudaStreamSynchronize(ctx->stream));
   geom G{};
-  G.nx = 1; G.ny = 1; G.num_cell = 1; G.max_cell = max_cell; G.dx = 1.; G.locked = 0;
+  G.nx = 1; G.ny = 1; G.num_cell = 1; G.max_cell = max_cell; G.dx = G.inv_dx = 1.; G.locked = 0;
   TRY(alloc_grid(ctx, max_cell));
   ctx->G = G;
   ctx->grid_kind = kind;
@@ -1178,7 +1194,7 @@ int batch_build_fused(mf_batch *b, int K) {
     // particles per pair block
     const int per = pair_bs / (c->P.precision == MF_PRECISION_MIXED ? 1 : pair64_lanes(c->N));
     const int blocks[4] = {c->scan_tiles, (c->N + BLOCK - 1) / BLOCK, (c->N + per - 1) / per,
-                           (int)std::max<long long>(1, (long long)sms * PLASTIC_BLOCKS_PER_SM * c->N / total_n)};
+                           c->P.plastic ? 1 + (int)std::max<long long>(1, (long long)sms * PLASTIC_BLOCKS_PER_SM * c->N / total_n) : 1};
     for (int m = 0; m < 4; ++m) first[(size_t)m * (n + 1) + k + 1] = first[(size_t)m * (n + 1) + k] + blocks[m];
   }
   for (int m = 0; m < 4; ++m) b->grid[m] = first[(size_t)m * (n + 1) + n];
@@ -1242,6 +1258,8 @@ int batch_build_fused(mf_batch *b, int K) {
     if (rc == MF_OK && P0.plastic)
       rc = P0.jc_model == MF_JC_TANH ? batch_kernel(b, kb_plastic<false>, b->grid[3], BLOCK, m_pl)
                                      : batch_kernel(b, kb_plastic<true>, b->grid[3], BLOCK, m_pl);
+    else if (rc == MF_OK)
+      rc = batch_kernel(b, kb_close, b->grid[3], BLOCK, m_pl);
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
@@ -1649,6 +1667,7 @@ int field_device_copy(mf_ctx *ctx, int field, void *dst_dev, const void *src_dev
     const size_t bytes = N * d.width * (d.is_int ? sizeof(int) : sizeof(double));
     e = to_ctx ? cudaMemcpyAsync(fp, src_dev, bytes, cudaMemcpyDeviceToDevice, st)
                : cudaMemcpyAsync(dst_dev, fp, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && to_ctx && touch_field(field)) e = mark_touch(ctx, st);
   }
   if (e != cudaSuccess) {
     ctx->last_cuda_err = (int)e;

@@ -150,12 +150,22 @@ static __global__ void __launch_bounds__(BS) kb_pse_mixed(batch_map M) {
   pse_mixed_system<BS>(s.P, s.D, b);
 }
 
-static __global__ void __launch_bounds__(FINISH_BLOCK, 2) kb_finish(batch_map M) {
+static __global__ void __launch_bounds__(FINISH_BLOCK, 4) kb_finish(batch_map M) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  finish_flat_body<true, false>(s.P, s.D, s.scan_tiles, b);
+  __shared__ finish_stage s_in;
+  finish_flat_body<true, false, false, true>(s.P, s.D, b, &s_in);
+}
+
+static __global__ void __launch_bounds__(BLOCK) kb_close(batch_map M) {
+  MF_PDL_WAIT();
+  MF_PDL_TRIGGER();
+  __shared__ batch_entry s;
+  __shared__ close_shared s_close;
+  batch_block(M, s);
+  close_step(s.P, s.D, finish_blocks(s.P.N), s_close);
 }
 
 template <bool PAIRED>
@@ -164,7 +174,8 @@ static __global__ void __launch_bounds__(BLOCK, 2) kb_plastic(batch_map M) {
   MF_PDL_TRIGGER();
   __shared__ batch_entry s;
   const blk b = batch_block(M, s);
-  plastic_body<PAIRED>(s.P, s.D, b);
+  __shared__ close_shared s_close;
+  plastic_body<PAIRED>(s.P, s.D, b, s_close);
 }
 
 }  // namespace mf

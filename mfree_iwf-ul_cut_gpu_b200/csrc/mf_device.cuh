@@ -18,6 +18,11 @@ constexpr unsigned FLAG_FIXED = 1u;
 constexpr unsigned FLAG_BLANKED = 2u;
 constexpr unsigned FLAG_TOOL = 4u;
 constexpr unsigned FLAG_NONFINITE = 8u;  // pair record holds a NaN/Inf (set per step)
+// The particle touched the tool at the end of the step that wrote the set: its contact and friction
+// forces there, and the contact normal at its array position, may be nonzero; without it they are
+// zero. So the few particles at the tool carry these 48 bytes, and the others neither read nor
+// write them. A host write of one of the three marks every particle.
+constexpr unsigned FLAG_TOUCH = 16u;
 
 // one FP64 pair record per particle: what a neighbour j contributes to the pair sums,
 // written once per step by the predictor kernel (16 doubles = one 128-byte line)
@@ -84,6 +89,7 @@ struct params {
 struct geom {
   int nx, ny, num_cell, max_cell;
   double bbmin_x, bbmin_y, bbmax_x, bbmax_y, dx;
+  double inv_dx;  // 1 / dx
   int locked;
   int pad;
 };
@@ -97,8 +103,8 @@ struct dev_status {
   unsigned long long steps;
   int max_cell_occupancy;
   int error_flags;
-  unsigned int force_ticket;
-  unsigned int scan_tile_counter;  // (unused: the cell scan takes no tile tickets)
+  unsigned int sorted_now;  // this step sorted (left by the finish kernel for the step's end)
+  unsigned int fused_now;   // this step's finish kernel ran the next step's predictor
   unsigned long long force_log_head;
   unsigned long long secant_iterations;
   unsigned long long sorts;  // cell-list sorts (every step, except with neighbour lists)

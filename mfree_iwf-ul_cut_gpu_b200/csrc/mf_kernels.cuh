@@ -61,10 +61,8 @@ struct dev_buffers {
   int *tsum_r, *tsum_w; // per-tile totals of the counts: read by this step's scan / added to by
                         // this step's counting for the next (two arrays, swapped every step)
   int *off;             // cell offsets (max_cell + 1)
-  double *partials;     // per-block partial sums (force / bbox); the force's group sums follow the
-                        // block partials (at [8 * number of block partials])
-  unsigned *ticket;     // last-block tickets: [0] force, [1] bbox, [2] tool wear
-  unsigned *gticket;    // per-group tickets of the force sums (one per FORCE_GROUP block partials)
+  double *partials;     // per-block partial sums (force / bbox)
+  unsigned *ticket;     // last-block tickets: [1] bbox, [2] tool wear
   double *force_log;    // FORCE_LOG_CAP x 2
   double *force_last;   // 2
   plastic_item *plastic_list;  // particles whose return map k_plastic runs (this step)
@@ -100,7 +98,7 @@ constexpr int BLOCK = 256;
 #define FINISH_BLOCK 256
 #endif
 // k_plastic: fixed grid of this many 256-thread blocks per SM over the plastic list
-constexpr int PLASTIC_BLOCKS_PER_SM = 4;
+constexpr int PLASTIC_BLOCKS_PER_SM = 3;
 #ifndef MF_PAIR_BLOCK
 #define MF_PAIR_BLOCK 128
 #endif
@@ -196,7 +194,7 @@ static __global__ void __launch_bounds__(BLOCK) k_bbox(int N, const double2 *__r
     return;  // keep the previous geometry; out-of-range hashes are clamped and counted
   }
   g.bbmin_x = bbmin_x; g.bbmin_y = bbmin_y; g.bbmax_x = bbmax_x; g.bbmax_y = bbmax_y;
-  g.dx = dx; g.nx = (int)nx; g.ny = (int)ny; g.num_cell = (int)nc;
+  g.dx = dx; g.inv_dx = 1. / dx; g.nx = (int)nx; g.ny = (int)ny; g.num_cell = (int)nc;
   *D.g = g;
 }
 
@@ -208,6 +206,16 @@ __device__ __forceinline__ void count_particle(int *count, int *tsum, int hsh) {
   const int tile = hsh / SCAN_TILE;
   const unsigned peers = __match_any_sync(__activemask(), tile);
   if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(&tsum[tile], __popc(peers));
+}
+
+// (int)(x / dx), the truncated quotient of grid.cu:34-51, without the division: away from whole
+// numbers the product with 1 / dx truncates to the same value (its error is below 4e-16 |x / dx|).
+__device__ __forceinline__ int cell_coordinate(double x, const geom &g) {
+  const double t = x * g.inv_dx;
+  const int i = __double2int_rz(t);
+  const double f = t - (double)i;
+  if (f > 1e-6 && f < 1. - 1e-6 && t < 1e9) return i;
+  return __double2int_rz(x / g.dx);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -224,8 +232,7 @@ static __global__ void __launch_bounds__(BLOCK) k_hash_count(int N, state_set A,
       hh = D.hash_cur[gid];  // blanked particles keep their previous hash (grid.cu:39-41)
     } else {
       double2 p = A.pos[gid];
-      int ix = __double2int_rz((p.x - g.bbmin_x) / g.dx);
-      int iy = __double2int_rz((p.y - g.bbmin_y) / g.dx);
+      const int ix = cell_coordinate(p.x - g.bbmin_x, g), iy = cell_coordinate(p.y - g.bbmin_y, g);
       hh = (long long)ix * (long long)g.ny + (long long)iy;
     }
     // outside [0, num_cell) the reference writes out of bounds; clamp and count instead
@@ -449,13 +456,16 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     B.rho[q] = rho;
     B.T[q] = T;
   }
+  // the set's contact forces of two steps ago at this place (staged, the reorder has copied the last
+  // step's there)
+  if (!P.staged && (B.flags[q] & FLAG_TOUCH)) B.fc[q] = B.ft[q] = make_double2(0., 0.);
   B.flags[q] = f;
 
   const double mass = P.phys.mass, K = P.phys.K;
   double prs = 0.;
   if (!tool) prs = P.eos_c0 * P.eos_c0 * (rho - P.phys.rho0);
   B.pp[q] = prs;
-  unsigned rf = f & (FLAG_BLANKED | FLAG_TOOL | FLAG_FIXED);
+  unsigned rf = f & (FLAG_BLANKED | FLAG_TOOL | FLAG_FIXED | FLAG_TOUCH);
   float fr[F_WIDTH];
   constexpr int fk[12] = {F_VX, F_VY, F_SXX, F_SXY, F_SYY, F_RXX, F_RXY, F_RYY, F_H, F_RHO, F_C, F_VOL};
   if (!MIXED || P.staged) {
@@ -531,13 +541,17 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
   }
 }
 
-// the last step's contact and friction forces of the particle at slot q (start-of-step slot p):
-// from the step's start set (the Rothlin grid does not gather ft: it stays in place,
+// the last step's contact and friction forces of the particle at slot q (start-of-step slot p, flags
+// f): from the step's start set (the Rothlin grid does not gather ft: it stays in place,
 // grid_gpu_rothlin.cu:138-250)
-__device__ __forceinline__ void prev_contact_forces(const params &P, const dev_buffers &D, int q, int p,
+__device__ __forceinline__ void prev_contact_forces(const params &P, const dev_buffers &D, int q, int p, unsigned f,
                                                     double2 &fc, double2 &ft) {
-  fc = D.A.fc[p];
-  ft = D.A.ft[P.grid_kind == MF_GRID_GREEN ? p : q];
+  fc = ft = make_double2(0., 0.);
+  if (f & FLAG_TOUCH) {
+    fc = D.A.fc[p];
+    ft = D.A.ft[p];
+  }
+  if (P.grid_kind != MF_GRID_GREEN) ft = D.A.ft[q];
 }
 
 // The rigid tool of this step: tool::update_tool (tool.cpp:211-221) with IEEE-rounded
@@ -650,7 +664,7 @@ __device__ __forceinline__ void reorder_body(const params &P, const dev_buffers 
     B.pos[q] = pos;
     B.rho[q] = rho;
     B.T[q] = T;
-    B.flags[q] = f;
+    B.flags[q] = f | FLAG_TOUCH;  // (the contact normals stay in place while the particles move)
     return;
   }
   predict_particle<MIXED>(P, D, B, q, hsh, pos, vel, S, rho, T, pos_t, vel_t, S_t, rho_t, T_t, f, h, sort);
@@ -933,7 +947,7 @@ __device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffer
     double2 pos_t = make_double2(__dmul_rn(m_eps, a.xt[0]), __dmul_rn(m_eps, a.xt[1]));
     if (!I.tool) {
       double2 fc, ft;
-      prev_contact_forces(P, D, q, p, fc, ft);
+      prev_contact_forces(P, D, q, p, fi, fc, ft);
       double ax = __dadd_rn(sdx, sdy), ay = __dadd_rn(sdz, sdw);
       if (fc.x != 0. || fc.y != 0. || ft.x != 0. || ft.y != 0.) {
         ax = __dadd_rn(ax, __dadd_rn(fc.x / mass, ft.x / mass));
@@ -1042,33 +1056,73 @@ static __global__ void __launch_bounds__(PAIR_BLOCK) k_pse(params P, dev_buffers
 
 // ---------------------------------------------------------------------------------------
 
+// What a thread of the finish kernel reads of its particle, staged in shared memory: asynchronous
+// copies of all of it are issued at once, without registers to land in, and the particle is worked
+// out of shared memory. (168 bytes a particle; the read of the start state through the permutation
+// is a gather on steps that sort.)
+enum : int { FI_POS = 0, FI_VEL, FI_POS_T, FI_VEL_T, FI_S01, FI_S23, FI_ST01, FI_ST23, FI_WIDE };
+enum : int { FI_RHO = 0, FI_T, FI_RHO_T, FI_T_T, FI_PP, FI_NARROW };
+struct finish_stage {
+  double2 wide[FI_WIDE][FINISH_BLOCK];
+  double narrow[FI_NARROW][FINISH_BLOCK];
+};
+__device__ __forceinline__ void copy_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async8(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void finish_fetch(const dev_buffers &D, finish_stage &s, int q, int p) {
+  const state_set &A = D.A, &B = D.B;
+  const int t = (int)threadIdx.x;
+  copy_async16(&s.wide[FI_POS][t], A.pos + p);
+  copy_async16(&s.wide[FI_VEL][t], A.vel + p);
+  copy_async16(&s.wide[FI_POS_T][t], B.pos_t + q);
+  copy_async16(&s.wide[FI_VEL_T][t], B.vel_t + q);
+  const double2 *S = reinterpret_cast<const double2 *>(A.S + p), *S_t = reinterpret_cast<const double2 *>(B.S_t + q);
+  copy_async16(&s.wide[FI_S01][t], S);
+  copy_async16(&s.wide[FI_S23][t], S + 1);
+  copy_async16(&s.wide[FI_ST01][t], S_t);
+  copy_async16(&s.wide[FI_ST23][t], S_t + 1);
+  copy_async8(&s.narrow[FI_RHO][t], A.rho + p);
+  copy_async8(&s.narrow[FI_T][t], A.T + p);
+  copy_async8(&s.narrow[FI_RHO_T][t], B.rho_t + q);
+  copy_async8(&s.narrow[FI_T_T][t], B.T_t + q);
+  copy_async8(&s.narrow[FI_PP][t], B.pp + q);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // Corrector .. invalidate for one particle (leap_frog.cu:68-92, actions_gpu.cu:135-162,
 // 226-349, tool_gpu.cu:151-221), in two phases that each load, update and store their own
 // fields: first velocity and position with the friction-heat input, contact, the kinematic
 // boundary conditions; then stress, density and temperature with the elastic test and the
 // thermal boundary condition. Fewer values are live at once than when every load is issued
 // first, so the kernel runs with fewer registers and more warps per SM. (eps_pl is not touched
-// here: the corrector does not change it, the return map in k_plastic does.) With FUSE_PRED and
+// here: the corrector does not change it, the return map in k_plastic does.) STAGED: the inputs
+// are in s (finish_fetch), else they are read from memory. With FUSE_PRED and
 // `fuse`, also the next step's predictor (neighbour lists, a step without a sort).
-template <bool FUSE_PRED, bool CONDUCT>
+template <bool FUSE_PRED, bool CONDUCT, bool STAGED>
 __device__ __forceinline__ void finish_particle_phased(const params &P, const dev_buffers &D,
-                                                       const mf_tool_state &TL, int q, double2 &pos_out,
-                                                       unsigned &f_out, double2 &fc_out, double2 &ft_out,
-                                                       unsigned &newly_blanked, bool &want_sort, bool identity,
-                                                       bool fuse) {
+                                                       const mf_tool_state &TL, const finish_stage *s, int q, int p,
+                                                       unsigned f, double2 &pos_out, unsigned &f_out,
+                                                       double2 &fc_out, double2 &ft_out, unsigned &newly_blanked,
+                                                       bool &want_sort, bool fuse) {
   const state_set &A = D.A;
   const state_set &B = D.B;
   const double dt = P.dt;
-  unsigned f = B.flags[q];
+  const int tid = (int)threadIdx.x;
   const bool blanked = f & FLAG_BLANKED;
   const bool tool = f & FLAG_TOOL;
   const bool fixed = f & FLAG_FIXED;
-  const int p = identity ? q : D.perm[q];
+  // the particle that was at this array position left a contact normal there
+  const unsigned f_here = A.flags[q];
   // phase 1: kinematics
-  double2 pos = A.pos[p], vel = A.vel[p];
-  double2 pos_t = B.pos_t[q], vel_t = B.vel_t[q];
+  double2 pos = STAGED ? s->wide[FI_POS][tid] : A.pos[p], vel = STAGED ? s->wide[FI_VEL][tid] : A.vel[p];
+  double2 pos_t = STAGED ? s->wide[FI_POS_T][tid] : B.pos_t[q], vel_t = STAGED ? s->wide[FI_VEL_T][tid] : B.vel_t[q];
   double2 fc, ft;
-  prev_contact_forces(P, D, q, p, fc, ft);
+  prev_contact_forces(P, D, q, p, f, fc, ft);
   if (!blanked) {  // correct (leap_frog.cu:68-92)
     pos.x = pos.x + dt * pos_t.x;
     pos.y = pos.y + dt * pos_t.y;
@@ -1103,7 +1157,7 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
       if (!inside) {
         fc = make_double2(0., 0.);
         ft = make_double2(0., 0.);
-        D.n[q] = make_double2(0., 0.);
+        if (f_here & FLAG_TOUCH) D.n[q] = make_double2(0., 0.);
       } else {
         const double dt2 = dt * dt;
         const double gN = (pos.x - cpx) * nx + (pos.y - cpy) * ny;
@@ -1155,13 +1209,25 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
   }
   B.pos[q] = pos;
   B.vel[q] = vel;
-  B.fc[q] = fc;
-  B.ft[q] = ft;
+  // (without a touch before or now both are zero, and so is what the set holds: predict_particle)
+  if (in_contact || (f & FLAG_TOUCH) || P.grid_kind != MF_GRID_GREEN) {
+    B.fc[q] = fc;
+    B.ft[q] = ft;
+  }
   // phase 2: stress, density, temperature
-  double4 S = A.S[p];
-  double rho = A.rho[p], T = A.T[p];
-  const double4 S_t = B.S_t[q];
-  const double rho_t = B.rho_t[q], T_t = B.T_t[q];
+  double4 S, S_t;
+  double rho, T, rho_t, T_t;
+  if (STAGED) {
+    const double2 a = s->wide[FI_S01][tid], b = s->wide[FI_S23][tid];
+    const double2 c = s->wide[FI_ST01][tid], d = s->wide[FI_ST23][tid];
+    S = make_double4(a.x, a.y, b.x, b.y);
+    S_t = make_double4(c.x, c.y, d.x, d.y);
+    rho = s->narrow[FI_RHO][tid]; T = s->narrow[FI_T][tid];
+    rho_t = s->narrow[FI_RHO_T][tid]; T_t = s->narrow[FI_T_T][tid];
+  } else {
+    S = A.S[p]; rho = A.rho[p]; T = A.T[p];
+    S_t = B.S_t[q]; rho_t = B.rho_t[q]; T_t = B.T_t[q];
+  }
   if (!blanked) {
     S.x = S.x + dt * S_t.x;
     S.y = S.y + dt * S_t.y;
@@ -1180,7 +1246,7 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
   // finish_particle, the rest in k_plastic
   bool elastic = false;
   if (P.plastic && !tool) {
-    const double pr = B.pp[q];
+    const double pr = STAGED ? s->narrow[FI_PP][tid] : B.pp[q];
     const double Sxx = S.x, Syy = S.z, Szz = S.w, Sxy = S.y;
     const double cxx = Sxx - pr, cyy = Syy - pr, czz = Szz - pr, cxy = Sxy;
     const double svm = (double)sqrtf(
@@ -1209,11 +1275,15 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
   B.S[q] = S;
   B.rho[q] = rho;
   B.T[q] = T;
+  // (a tool particle leaves the normal at its array position as it is: it keeps the mark of it)
+  unsigned fn = f;
+  if (P.has_tool && tool) fn = f | (f_here & FLAG_TOUCH);
+  else if (P.has_tool) fn = in_contact ? f | FLAG_TOUCH : f & ~FLAG_TOUCH;
   if (invalid) {  // invalidate (actions_gpu.cu:317-349)
-    f |= FLAG_BLANKED;
+    fn |= FLAG_BLANKED;
     newly_blanked += 1u;
-    B.flags[q] = f;
   }
+  if (fn != f) B.flags[q] = f = fn;
   if (far && !(f & FLAG_BLANKED)) want_sort = true;
   if (FUSE_PRED && fuse) {
     // neighbour lists, a step without a sort: the next step keeps this order, so its predictor
@@ -1239,9 +1309,7 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
 // of fc.x, fc.y, ft.x, ft.y) in a fixed two-level tree: the partials of each group of
 // FORCE_GROUP consecutive blocks summed by one warp (lane l takes the group's l-th partial,
 // then a shuffle tree), then the group sums by one warp (lane l takes groups l, l + 32, ... in
-// order, then the same tree). In the flat finish kernel the block that completes a group sums
-// it and the block that completes the last group sums the groups: each step of the tree is one
-// load per lane and a shuffle tree, so no block waits long and no warp walks a long chain.
+// order, then the same tree).
 constexpr int FORCE_GROUP = 32;
 
 __device__ __forceinline__ void ksum4_shuffle_tree(ksum r[4]) {
@@ -1252,48 +1320,51 @@ __device__ __forceinline__ void ksum4_shuffle_tree(ksum r[4]) {
     }
 }
 
-// lane 0: the sum of group g of the nb block partials (read through L2: other blocks wrote them
-// before their fence and ticket)
-__device__ __forceinline__ void force_group_sum(const double *partials, int g, int nb, ksum r[4]) {
-  const int b = g * FORCE_GROUP + (int)lane_id();
-  for (int k = 0; k < 4; ++k) r[k] = ksum{0., 0.};
-  if (b < nb) {
-    const double2 *pr = reinterpret_cast<const double2 *>(partials) + (size_t)b * 4;
-    for (int k = 0; k < 4; ++k) {
-      const double2 v = __ldcg(pr + k);
-      r[k] = ksum{v.x, v.y};
+// The end of a step, by one block of BLOCK threads after the finish kernel (nb block partials): the
+// tool force (report_force, output.cu:31-39: contact plus friction force) into force_last and the
+// log, the step's counters and the next step's sort decision. It runs beside the return map, as
+// the last block of its launch: closed by the finish kernel's own last block, through tickets, it
+// was that kernel's tail (two fences, two tickets and two trees in a row). Groups without contact
+// (nearly all) skip their tree: {+0, +0} is what the sums give for zeros.
+constexpr int CLOSE_GROUPS = 64;  // groups at a time
+struct close_shared {
+  ksum group[CLOSE_GROUPS][4];
+};
+__device__ __forceinline__ void close_step(const params &P, const dev_buffers &D, int nb, close_shared &s) {
+  const int warp = (int)threadIdx.x >> 5, lane = (int)lane_id();
+  const int ng = (nb + FORCE_GROUP - 1) / FORCE_GROUP;
+  const double2 *pr = reinterpret_cast<const double2 *>(D.partials);
+  ksum total[4];
+  for (int k = 0; k < 4; ++k) total[k] = ksum{0., 0.};
+  for (int g0 = 0; g0 < ng; g0 += CLOSE_GROUPS) {
+    const int gn = min(CLOSE_GROUPS, ng - g0);
+    for (int g = warp; g < gn; g += BLOCK / 32) {
+      const int b = (g0 + g) * FORCE_GROUP + lane;
+      ksum r[4];
+      for (int k = 0; k < 4; ++k) r[k] = ksum{0., 0.};
+      bool nz = false;
+      if (b < nb) {
+        for (int k = 0; k < 4; ++k) {
+          const double2 v = __ldcg(pr + (size_t)b * 4 + k);
+          r[k] = ksum{v.x, v.y};
+          nz = nz || v.x != 0. || v.y != 0.;  // (true for a NaN)
+        }
+      }
+      if (__any_sync(0xffffffffu, nz)) ksum4_shuffle_tree(r);
+      if (lane == 0)
+        for (int k = 0; k < 4; ++k) s.group[g][k] = r[k];
     }
+    __syncthreads();
+    if (warp == 0)
+      for (int g = lane; g < gn; g += 32)
+        for (int k = 0; k < 4; ++k) ksum_merge(total[k], s.group[g][k]);
+    __syncthreads();
   }
-  ksum4_shuffle_tree(r);
-}
-
-__device__ __forceinline__ void store_ksum4(double *dst, const ksum r[4]) {
-  for (int k = 0; k < 4; ++k) {
-    dst[2 * k] = r[k].s;
-    dst[2 * k + 1] = r[k].c;
-  }
-}
-
-// lane 0: the sum of the ng group sums
-__device__ __forceinline__ void force_final_sum(const double *gsums, int ng, ksum r[4]) {
-  for (int k = 0; k < 4; ++k) r[k] = ksum{0., 0.};
-  const double2 *pr = reinterpret_cast<const double2 *>(gsums);
-  for (int g = (int)lane_id(); g < ng; g += 32)
-    for (int k = 0; k < 4; ++k) {
-      const double2 v = __ldcg(pr + (size_t)g * 4 + k);
-      ksum x{v.x, v.y};
-      ksum_merge(r[k], x);
-    }
-  ksum4_shuffle_tree(r);
-}
-
-// lane 0 of the warp that finished the sum: report_force (output.cu:31-39: contact plus
-// friction force) into force_last and the log, the step's counters, the tickets re-armed.
-// `predicted`: the next step's predictor ran in this kernel.
-__device__ __forceinline__ void force_close_step(const params &P, const dev_buffers &D, const ksum r[4],
-                                                 bool predicted, bool sorted) {
-  const double Fx = (r[0].s + r[0].c) + (r[2].s + r[2].c);
-  const double Fy = (r[1].s + r[1].c) + (r[3].s + r[3].c);
+  if (warp != 0) return;
+  ksum4_shuffle_tree(total);
+  if (lane != 0) return;
+  const double Fx = (total[0].s + total[0].c) + (total[2].s + total[2].c);
+  const double Fy = (total[1].s + total[1].c) + (total[3].s + total[3].c);
   D.force_last[0] = Fx;
   D.force_last[1] = Fy;
   const unsigned long long hd = D.st->force_log_head;
@@ -1301,44 +1372,68 @@ __device__ __forceinline__ void force_close_step(const params &P, const dev_buff
   D.force_log[2 * (hd % FORCE_LOG_CAP) + 1] = Fy;
   D.st->force_log_head = hd + 1;
   D.st->steps += 1;
-  if (P.verlet) {  // every particle is checked: the next step sorts if one asked for it
+  if (P.verlet) {  // every particle was checked: the next step sorts if one asked for it
     D.st->sort_now = D.st->want_sort;
     D.st->want_sort = 0u;
-    D.st->predicted = predicted ? 1u : 0u;
+    D.st->predicted = D.st->fused_now;
   }
-  D.st->sorted_prev = sorted ? 1u : 0u;
-  D.ticket[0] = 0u;
+  D.st->sorted_prev = D.st->sorted_now;
 }
 
-// Corrector .. invalidate for all particles plus the tool force (output.cu:31-39): one thread
-// per particle, one block per FINISH_BLOCK consecutive particles; the force sums per warp, then
-// the block's warps in order, then the two-level group tree. With FUSE_HASH (locked grid) also
+__device__ __forceinline__ int finish_blocks(int N) { return (N + FINISH_BLOCK - 1) / FINISH_BLOCK; }
+
+// the end of a step without plasticity (no return map to run beside)
+static __global__ void __launch_bounds__(BLOCK) k_close(params P, dev_buffers D) {
+  MF_PDL_WAIT();
+  MF_PDL_TRIGGER();
+  __shared__ close_shared s_close;
+  close_step(P, D, finish_blocks(P.N), s_close);
+}
+
+// Corrector .. invalidate for all particles plus each block's tool force (output.cu:31-39): one
+// thread per particle, one block per FINISH_BLOCK consecutive particles; the force sums per warp,
+// then the block's warps in order. With FUSE_HASH (locked grid) also
 // the next step's hash and count; with FUSE_PRED the next step's predictor on list steps
-// without a sort (MF_OPT_FUSED_PREDICTOR). (A persistent variant of the fused kernel, blocks
-// taking 256-particle chunks from a counter at 128 registers, measured 44 against these 38 us
-// and gave the same bits.)
+// without a sort (MF_OPT_FUSED_PREDICTOR).
+// Bound by the latency of its loads: their asynchronous copies into shared memory (44 KB a block) put
+// every one of a block's in flight at once, where two phases of loads at 80 registers and 3 blocks
+// per SM waited twice; at 4 blocks per SM (64 registers) the ~177k-particle grid also runs in fewer
+// rounds. Finish + return map stage in us (launches included), before / so: 6,149 particles 19.5 /
+// 17.4; 45,052 21.5 / 17.4; 176,695 29.7 / 23.6; 577,555 68.6 / 55.5; at 3 blocks per SM (80
+// registers) 17.4, 17.4, 25.6, 58.4, at 5 (48) 19.5, 21.5, 25.6, 60.5. (A persistent variant of the
+// fused kernel, blocks taking 256-particle chunks from a counter at 128 registers, measured 44
+// against 38 us and gave the same bits.)
 #ifndef FINISH_FLAT_MIN_BLOCKS
-#define FINISH_FLAT_MIN_BLOCKS 3
+#define FINISH_FLAT_MIN_BLOCKS 4
 #endif
-template <bool FUSE_HASH, bool FUSE_PRED, bool CONDUCT = false>
-__device__ __forceinline__ void finish_flat_body(const params &P, const dev_buffers &D,
-                                                                                    int num_scan_tiles, blk bk) {
+template <bool FUSE_HASH, bool FUSE_PRED, bool CONDUCT, bool STAGED>
+__device__ __forceinline__ void finish_flat_body(const params &P, const dev_buffers &D, blk bk, finish_stage *s_in) {
   __shared__ mf_tool_state s_tool;
   __shared__ ksum sm[FINISH_BLOCK / 32][4];
   __shared__ unsigned smc[FINISH_BLOCK / 32][4];
-  if (P.has_tool) tool_load_shared(s_tool, D);
   const int q = bk.x * FINISH_BLOCK + threadIdx.x;
-  const bool identity = P.verlet && !*(volatile unsigned *)&D.st->sort_now;
+  const bool identity = P.verlet && !D.st->sort_now;
   const bool fuse = FUSE_PRED && identity && P.fuse;  // the next step's predictor runs here too
-  (void)num_scan_tiles;
+  unsigned f = 0u;
+  int p = q;
+  if (q < P.N) {
+    f = D.B.flags[q];
+    if (!identity) p = D.perm[q];
+    if (STAGED) finish_fetch(D, *s_in, q, p);
+  }
+  if (bk.x == 0 && threadIdx.x == 0) {
+    D.st->sorted_now = identity ? 0u : 1u;
+    D.st->fused_now = fuse ? 1u : 0u;
+  }
+  if (P.has_tool) tool_load_shared(s_tool, D);  // while the copies are under way
+  if (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");  // (each thread reads its own)
   double2 fc = make_double2(0., 0.), ft = make_double2(0., 0.);
   unsigned newly_blanked = 0, blanked_now = 0, oog = 0;
   bool want_sort = false;
   if (q < P.N) {
     double2 pos;
-    unsigned f;
-    finish_particle_phased<FUSE_PRED, CONDUCT>(P, D, s_tool, q, pos, f, fc, ft, newly_blanked, want_sort, identity,
-                                               fuse);
+    finish_particle_phased<FUSE_PRED, CONDUCT, STAGED>(P, D, s_tool, s_in, q, p, f, pos, f, fc, ft, newly_blanked,
+                                                       want_sort, fuse);
     blanked_now = (f & FLAG_BLANKED) ? 1u : 0u;
     if (FUSE_HASH) {  // compute_hashes of the next step (grid.cu:34-51)
       const geom g = *D.g;
@@ -1346,8 +1441,8 @@ __device__ __forceinline__ void finish_flat_body(const params &P, const dev_buff
       if (f & FLAG_BLANKED) {
         hh = D.hash_cur[q];
       } else {
-        const int ix = __double2int_rz(P.verlet ? (pos.x - g.bbmin_x) * (1. / g.dx) : (pos.x - g.bbmin_x) / g.dx);
-        const int iy = __double2int_rz(P.verlet ? (pos.y - g.bbmin_y) * (1. / g.dx) : (pos.y - g.bbmin_y) / g.dx);
+        const int ix = P.verlet ? __double2int_rz((pos.x - g.bbmin_x) * g.inv_dx) : cell_coordinate(pos.x - g.bbmin_x, g);
+        const int iy = P.verlet ? __double2int_rz((pos.y - g.bbmin_y) * g.inv_dx) : cell_coordinate(pos.y - g.bbmin_y, g);
         hh = (long long)ix * (long long)g.ny + (long long)iy;
       }
       if (hh < 0) { hh = 0; oog = 1; }
@@ -1362,24 +1457,16 @@ __device__ __forceinline__ void finish_flat_body(const params &P, const dev_buff
   const bool nz = fc.x != 0. || fc.y != 0. || ft.x != 0. || ft.y != 0.;
   const int w = threadIdx.x >> 5;
   if (__any_sync(0xffffffffu, nz)) {
-    ksum fcx{0., 0.}, fcy{0., 0.}, ftx{0., 0.}, fty{0., 0.};
-    ksum_add(fcx, fc.x);
-    ksum_add(fcy, fc.y);
-    ksum_add(ftx, ft.x);
-    ksum_add(fty, ft.y);
-    for (int o = 16; o > 0; o >>= 1) {
-      ksum a{__shfl_down_sync(0xffffffffu, fcx.s, o), __shfl_down_sync(0xffffffffu, fcx.c, o)};
-      ksum b{__shfl_down_sync(0xffffffffu, fcy.s, o), __shfl_down_sync(0xffffffffu, fcy.c, o)};
-      ksum c{__shfl_down_sync(0xffffffffu, ftx.s, o), __shfl_down_sync(0xffffffffu, ftx.c, o)};
-      ksum d{__shfl_down_sync(0xffffffffu, fty.s, o), __shfl_down_sync(0xffffffffu, fty.c, o)};
-      ksum_merge(fcx, a); ksum_merge(fcy, b); ksum_merge(ftx, c); ksum_merge(fty, d);
-    }
-    if (lane_id() == 0) {
-      sm[w][0] = fcx; sm[w][1] = fcy; sm[w][2] = ftx; sm[w][3] = fty;
-    }
+    ksum r[4] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
+    ksum_add(r[0], fc.x);
+    ksum_add(r[1], fc.y);
+    ksum_add(r[2], ft.x);
+    ksum_add(r[3], ft.y);
+    ksum4_shuffle_tree(r);
+    if (lane_id() == 0)
+      for (int k = 0; k < 4; ++k) sm[w][k] = r[k];
   } else if (lane_id() == 0) {
-    const ksum z{0., 0.};
-    sm[w][0] = z; sm[w][1] = z; sm[w][2] = z; sm[w][3] = z;
+    for (int k = 0; k < 4; ++k) sm[w][k] = ksum{0., 0.};
   }
   const unsigned nb = __reduce_add_sync(0xffffffffu, newly_blanked);
   const unsigned nbl = __reduce_add_sync(0xffffffffu, blanked_now);
@@ -1388,63 +1475,33 @@ __device__ __forceinline__ void finish_flat_body(const params &P, const dev_buff
   if (lane_id() == 0) {
     smc[w][0] = nb; smc[w][1] = nbl; smc[w][2] = noog; smc[w][3] = nws;
   }
-  const bool block_nz = __syncthreads_or(nz);  // sm and smc complete
-  // warp 0 closes the block (the block's sums into its partial, the counters, the ticket) and,
-  // in the last block, the step; the other warps are done
-  if (threadIdx.x >= 32) return;
-  unsigned is_last = 0u;
-  if (threadIdx.x == 0) {
-    ksum r[4] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
-    if (block_nz) {
-      for (int k = 0; k < 4; ++k) r[k] = sm[0][k];
-      for (int v = 1; v < FINISH_BLOCK / 32; ++v)
-        for (int k = 0; k < 4; ++k) ksum_merge(r[k], sm[v][k]);
-    }
-    for (int k = 0; k < 4; ++k) {
-      D.partials[(size_t)bk.x * 8 + 2 * k] = r[k].s;
-      D.partials[(size_t)bk.x * 8 + 2 * k + 1] = r[k].c;
-    }
+  const bool block_any = __syncthreads_or(nz || nb || nbl || noog || nws);  // sm and smc complete
+  if (threadIdx.x != 0) return;
+  ksum r[4] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
+  if (block_any) {
+    for (int k = 0; k < 4; ++k) r[k] = sm[0][k];
     unsigned long long cnt[3] = {smc[0][0], smc[0][1], smc[0][2]};
     unsigned ws = smc[0][3];
     for (int v = 1; v < FINISH_BLOCK / 32; ++v) {
+      for (int k = 0; k < 4; ++k) ksum_merge(r[k], sm[v][k]);
       for (int k = 0; k < 3; ++k) cnt[k] += smc[v][k];
       ws |= smc[v][3];
     }
-    if (ws) D.st->want_sort = 1u;  // (before the fence and the ticket below)
+    if (ws) D.st->want_sort = 1u;
     if (cnt[0]) atomicAdd(&D.st->newly_blanked, cnt[0]);
     if (cnt[1]) atomicAdd(&D.st->blanked, cnt[1]);
     if (cnt[2]) atomicAdd(&D.st->out_of_grid, cnt[2]);
-    __threadfence();
-    const int g = bk.x / FORCE_GROUP;
-    const int gsize = min(FORCE_GROUP, bk.n - g * FORCE_GROUP);
-    is_last = atomicAdd(&D.gticket[g], 1u) == (unsigned)(gsize - 1) ? 1u : 0u;
   }
-  if (!__shfl_sync(0xffffffffu, is_last, 0)) return;
-  // this block completed its group: the group's sum, then the group ticket
-  __threadfence();
-  const int g = bk.x / FORCE_GROUP;
-  const int ng = (bk.n + FORCE_GROUP - 1) / FORCE_GROUP;
-  double *gsums = D.partials + (size_t)bk.n * 8;
-  ksum r[4];
-  force_group_sum(D.partials, g, bk.n, r);
-  unsigned last = 0u;
-  if (lane_id() == 0) {
-    store_ksum4(gsums + (size_t)g * 8, r);
-    D.gticket[g] = 0u;
-    __threadfence();
-    last = atomicAdd(&D.ticket[0], 1u) == (unsigned)(ng - 1) ? 1u : 0u;
-  }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
-  __threadfence();
-  force_final_sum(gsums, ng, r);
-  if (lane_id() == 0) force_close_step(P, D, r, fuse, !identity);
+  double2 *out = reinterpret_cast<double2 *>(D.partials) + (size_t)bk.x * 4;
+  for (int k = 0; k < 4; ++k) out[k] = make_double2(r[k].s, r[k].c);
 }
 
 template <bool FUSE_HASH, bool FUSE_PRED, bool CONDUCT = false>
-__global__ void __launch_bounds__(FINISH_BLOCK, FINISH_FLAT_MIN_BLOCKS) k_finish_flat(params P, dev_buffers D, int num_scan_tiles) {
+__global__ void __launch_bounds__(FINISH_BLOCK, FINISH_FLAT_MIN_BLOCKS) k_finish_flat(params P, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
-  finish_flat_body<FUSE_HASH, FUSE_PRED, CONDUCT>(P, D, num_scan_tiles, grid_blk());
+  __shared__ finish_stage s_in;
+  finish_flat_body<FUSE_HASH, FUSE_PRED, CONDUCT, true>(P, D, grid_blk(), &s_in);
 }
 
 // JC plasticity (actions_gpu.cu:226-285) for the particles the finish kernel listed: the
@@ -1510,8 +1567,13 @@ __device__ __forceinline__ double solve_secant_pair(const mf_joco_constants &jc,
   }
 }
 
+// The last block of the launch (bk.n - 1) ends the step meanwhile (close_step).
 template <bool PAIRED>
-__device__ __forceinline__ void plastic_body(const params &P, const dev_buffers &D, blk bk) {
+__device__ __forceinline__ void plastic_body(const params &P, const dev_buffers &D, blk bk, close_shared &s_close) {
+  if (bk.x == bk.n - 1) {
+    close_step(P, D, finish_blocks(P.N), s_close);
+    return;
+  }
   __shared__ mf_joco_constants s_jc;  // by reference into the out-of-line functions
   __shared__ unsigned long long s_cnt[BLOCK / 32][2];
   if (threadIdx.x == 0) s_jc = P.joco;
@@ -1522,12 +1584,12 @@ __device__ __forceinline__ void plastic_body(const params &P, const dev_buffers 
   const double dt = P.dt, mu = P.phys.G;
   // neighbour lists: the finish kernel ran the next step's predictor; redone here where the
   // return map changes the state
-  const bool fuse = P.verlet && D.st->predicted;
+  const bool fuse = P.verlet && D.st->fused_now;
   constexpr unsigned LANES = PAIRED ? 2u : 1u;
   const unsigned sub = PAIRED ? (lane_id() & 1u) : 0u;
   const unsigned pmask = PAIRED ? (0x3u << (lane_id() & ~1u)) : 0xffffffffu;
   unsigned capped = 0u, iters_sum = 0u;
-  const unsigned stride = bk.n * blockDim.x / LANES;
+  const unsigned stride = (bk.n - 1) * blockDim.x / LANES;
   for (unsigned i = (bk.x * blockDim.x + threadIdx.x) / LANES; i < n; i += stride) {
     const plastic_item it = D.plastic_list[i];
     const int q = it.q;
@@ -1614,7 +1676,8 @@ template <bool PAIRED>
 static __global__ void __launch_bounds__(BLOCK, PLASTIC_BLOCKS_PER_SM) k_plastic(params P, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
-  plastic_body<PAIRED>(P, D, grid_blk());
+  __shared__ close_shared s_close;
+  plastic_body<PAIRED>(P, D, grid_blk(), s_close);
 }
 
 // Usui tool wear rate (tool_wear.cu:20-64) on the current state, on the device instead of

@@ -312,7 +312,7 @@ __device__ __forceinline__ void mixed_end(const params &P, const dev_buffers &D,
     B.S_t[q] = make_double4(tx, ty, tz, tw);
     B.rho_t[q] = -(double)rhoi * (double)(vdx + vdw);
     double2 fc, ft;
-    prev_contact_forces(P, D, q, p, fc, ft);
+    prev_contact_forces(P, D, q, p, B.flags[q], fc, ft);
     const double2 vp = B.vel[q];
     double2 vel_t = make_double2((double)(vtx + (sdx + sdy)), (double)(vty + (sdz + sdw)));
     if (fc.x != 0. || fc.y != 0. || ft.x != 0. || ft.y != 0.) {  // (few particles touch the tool)

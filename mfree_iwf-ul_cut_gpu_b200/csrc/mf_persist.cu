@@ -114,7 +114,9 @@ __device__ __forceinline__ void persist_phase(const batch_map &m, int nvb, batch
 
 __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args A) {
   __shared__ batch_entry s;
-  __shared__ unsigned s_list[mixed_shared<PERSIST_BLOCK>::WORDS];
+  __shared__ __align__(16) unsigned s_list[mixed_shared<PERSIST_BLOCK>::WORDS];
+  static_assert(sizeof(close_shared) <= sizeof(s_list), "the phases share it");
+  close_shared &s_close = *reinterpret_cast<close_shared *>(s_list);
   for (int st = 0; st < A.K; ++st) {
     const batch_entry *ent = A.e + (size_t)(st & 1) * A.n;
     const batch_map m_scan{ent, A.first, A.n}, m_256{ent, A.first + (A.n + 1), A.n},
@@ -131,13 +133,15 @@ __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args 
       persist_phase(m_pair, A.grid[2], s, [&](blk b) { pse_mixed_system<PERSIST_BLOCK>(s.P, s.D, b); });
       if (!persist_sync(A)) return;
     }
-    persist_phase(m_256, A.grid[1], s, [&](blk b) { finish_flat_body<true, false>(s.P, s.D, s.scan_tiles, b); });
+    persist_phase(m_256, A.grid[1], s, [&](blk b) { finish_flat_body<true, false, false, false>(s.P, s.D, b, nullptr); });
     if (!persist_sync(A)) return;
     if (A.plastic) {
-      if (A.paired) persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<true>(s.P, s.D, b); });
-      else persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<false>(s.P, s.D, b); });
-      if (st + 1 < A.K && !persist_sync(A)) return;
+      if (A.paired) persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<true>(s.P, s.D, b, s_close); });
+      else persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<false>(s.P, s.D, b, s_close); });
+    } else {
+      persist_phase(m_pl, A.grid[3], s, [&](blk b) { close_step(s.P, s.D, finish_blocks(s.P.N), s_close); });
     }
+    if (st + 1 < A.K && !persist_sync(A)) return;
   }
 }
 
