@@ -24,7 +24,8 @@ __device__ __forceinline__ bool f_nonfinite(const float4 &b0) { return __float_a
 
 // the i particle's values and the pair sums of one thread
 struct mixed_i {
-  float x, y, row, vx, vy, sxx, sxy, syy, Rxx, Rxy, Ryy, h, rho, c, T;  // row: cell row + 1
+  float x, y, row, sxy, Rxy, h, rho, c, T;  // row: cell row + 1
+  float2 nv, sd, Rd;                        // (-vx, -vy), (sxx, syy), (Rxx, Ryy)
   float h1, fourh2;
   // the spline's coefficients: W / W(dp) for q > 1 (w_out (2 - q)^6) and q <= 1 (w_in (1 - 1.5 q^2 +
   // 0.75 q^3)), (dW/dr) / r for q > 1 (d_out (2 - q)^2 / r) and q <= 1 (d_in (1 - 0.75 q))
@@ -34,8 +35,10 @@ struct mixed_i {
 // The constant factors of a sum are applied once at the end: the stress sums without the mass, the
 // viscosity sums without -2 mass, XSPH without 2 mass eps W(dp), the Brookshaw sum without its factor 2.
 struct mixed_acc {
-  float vdx, vdy, vdz, vdw;
-  float sdx, sdy, sdz, sdw;
+  float2 v14;  // (vdx, vdw)
+  float vdy, vdz;
+  float2 s14;  // (sdx, sdw)
+  float sdy, sdz;
   float vtx, vty, xtx, xty;
   float T_lapl;
 };
@@ -57,11 +60,13 @@ __device__ __forceinline__ float offset_y(const mixed_i &I, const float4 &b0, fl
 
 // One neighbour j (records b0..b3) of particle i at offset (xij, yij): the reference's cubic spline
 // (kernels.cuh:30-70; its value (2 - q)^6 / 4 for q > 1 is sic), both branches evaluated and selected,
-// with the constants folded into the coefficients (1 / r cancels for q <= 1). In scalars, every
-// multiply-add written out: sm_100's packed pairs (two multiply-adds an issue) save issues only where
-// both operands already lie in register pairs; the moves that built pairs of duplicated factors cost
-// the ALU pipe more than the packed arithmetic gave back (1,100 against 1,770 integer instructions a
-// particle at ~577k particles).
+// with the constants folded into the coefficients (1 / r cancels for q <= 1). SELECT: both branches
+// evaluated and selected (the list form, 48.2 against 50.1 us at 176,695 particles; the window form's
+// lanes take the branches together more often and lose by it, 201 against 191 us at 577,555). Every
+// multiply-add is written out. Packed pairs (two multiply-adds an issue) stand only where both
+// operands already lie in register pairs, as words of a record or sums side by side: the moves that
+// built pairs of duplicated factors cost the ALU pipe more than they gave back (1,100 against 1,770
+// integer instructions a particle at 577,555; 24-system batch 181.5 all scalar, 179.3 us so).
 template <bool SELECT>
 __device__ __forceinline__ void mixed_interact(const mixed_i &I, const mixed_const &K, mixed_acc &a, float xij,
                                                float yij, const float4 &b0, const float4 &b1, const float4 &b2,
@@ -92,18 +97,18 @@ __device__ __forceinline__ void mixed_interact(const mixed_i &I, const mixed_con
   const float wx = __fmul_rn(dwr, xij), wy = __fmul_rn(dwr, yij);
   const float volj = b3.z;
   if (I.mech && !f_tool(b0)) {
-    const float dvx = b1.x - I.vx, dvy = b1.y - I.vy;
+    const float2 dv = __fadd2_rn(make_float2(b1.x, b1.y), I.nv);
+    const float dvx = dv.x, dvy = dv.y;
+    const float2 w2v = make_float2(wx, wy);
     const float ax = __fmul_rn(dvx, volj), ay = __fmul_rn(dvy, volj);
-    a.vdx = fmaf(ax, wx, a.vdx);
+    a.v14 = __ffma2_rn(make_float2(ax, ay), w2v, a.v14);
     a.vdy = fmaf(ax, wy, a.vdy);
     a.vdz = fmaf(ay, wx, a.vdz);
-    a.vdw = fmaf(ay, wy, a.vdw);
     const float w2 = __fmul_rn(w, w), fab = __fmul_rn(w2, w2);
-    const float sxx = fmaf(fab, I.Rxx + b2.z, I.sxx + b2.x);
-    const float syy = fmaf(fab, I.Ryy + b2.w, I.syy + b2.y);
+    const float2 Rs = __fadd2_rn(I.Rd, make_float2(b2.z, b2.w)), ss = __fadd2_rn(I.sd, make_float2(b2.x, b2.y));
+    const float2 sd2 = make_float2(fmaf(fab, Rs.x, ss.x), fmaf(fab, Rs.y, ss.y));
     const float sxy = fmaf(fab, I.Rxy + b1.w, I.sxy + b1.z);
-    a.sdx = fmaf(sxx, wx, a.sdx);
-    a.sdw = fmaf(syy, wy, a.sdw);
+    a.s14 = __ffma2_rn(sd2, w2v, a.s14);
     a.sdz = fmaf(sxy, wx, a.sdz);
     a.sdy = fmaf(sxy, wy, a.sdy);
     const float nvr = fmaf(dvx, xij, __fmul_rn(dvy, yij));  // -v_ij . x_ij
@@ -262,9 +267,9 @@ __device__ __forceinline__ bool mixed_begin(const params &P, const dev_buffers &
   I.nonfinite = f_nonfinite(a0);
   I.mech = !tool_i;
   I.x = a0.x; I.y = a0.y; I.row = fabsf(a0.z); I.h = fabsf(a0.w);
-  I.vx = a1.x; I.vy = a1.y;
-  I.sxx = a2.x; I.syy = a2.y; I.sxy = a1.z;
-  I.Rxx = a2.z; I.Ryy = a2.w; I.Rxy = a1.w;
+  I.nv = make_float2(-a1.x, -a1.y);
+  I.sd = make_float2(a2.x, a2.y); I.sxy = a1.z;
+  I.Rd = make_float2(a2.z, a2.w); I.Rxy = a1.w;
   I.rho = a3.x; I.c = a3.y; I.T = I.thermal ? a3.w : 0.f;
   // the spline's constants from the FP64 smoothing length, rounded once: an error of the rounded h
   // would enter every gradient four times over, all with the same sign
@@ -284,8 +289,8 @@ __device__ __forceinline__ void mixed_end(const params &P, const dev_buffers &D,
                                           const mixed_acc &acc, double thermal_alpha) {
   const float mass = (float)P.phys.mass;
   const float m2 = 2.f * mass, m_eps = (float)P.corr.xspheps * m2 * (float)P.corr.wdeltap;
-  const float vdx = acc.vdx, vdy = acc.vdy, vdz = acc.vdz, vdw = acc.vdw;
-  const float sdx = mass * acc.sdx, sdy = mass * acc.sdy, sdz = mass * acc.sdz, sdw = mass * acc.sdw;
+  const float vdx = acc.v14.x, vdy = acc.vdy, vdz = acc.vdz, vdw = acc.v14.y;
+  const float sdx = mass * acc.s14.x, sdy = mass * acc.sdy, sdz = mass * acc.sdz, sdw = mass * acc.s14.y;
   const float vtx = -m2 * acc.vtx, vty = -m2 * acc.vty;
   const float xtx = m_eps * acc.xtx, xty = m_eps * acc.xty, T_lapl = 2.f * acc.T_lapl;
   const bool mech_i = I.mech, thermal = I.thermal;
@@ -349,13 +354,13 @@ struct mixed_shared {
 };
 
 __device__ __forceinline__ void acc_add(mixed_acc &a, const mixed_acc &b) {
-  a.vdx += b.vdx; a.vdy += b.vdy; a.vdz += b.vdz; a.vdw += b.vdw;
-  a.sdx += b.sdx; a.sdy += b.sdy; a.sdz += b.sdz; a.sdw += b.sdw;
+  a.v14.x += b.v14.x; a.vdy += b.vdy; a.vdz += b.vdz; a.v14.y += b.v14.y;
+  a.s14.x += b.s14.x; a.sdy += b.sdy; a.sdz += b.sdz; a.s14.y += b.s14.y;
   a.vtx += b.vtx; a.vty += b.vty; a.xtx += b.xtx; a.xty += b.xty;
   a.T_lapl += b.T_lapl;
 }
 __device__ __forceinline__ void acc_zero(mixed_acc &a) {
-  a.vdx = a.vdy = a.vdz = a.vdw = a.sdx = a.sdy = a.sdz = a.sdw = 0.f;
+  a.v14 = a.s14 = make_float2(0.f, 0.f); a.vdy = a.vdz = a.sdy = a.sdz = 0.f;
   a.vtx = a.vty = a.xtx = a.xty = a.T_lapl = 0.f;
 }
 
@@ -573,10 +578,10 @@ __device__ __forceinline__ void pair_mixed_body(const params &P, const dev_buffe
 #pragma unroll
     for (int r = 1; r < G; ++r) {
       mixed_acc o;
-      o.vdx = __shfl_down_sync(0xffffffffu, own.vdx, r); o.vdy = __shfl_down_sync(0xffffffffu, own.vdy, r);
-      o.vdz = __shfl_down_sync(0xffffffffu, own.vdz, r); o.vdw = __shfl_down_sync(0xffffffffu, own.vdw, r);
-      o.sdx = __shfl_down_sync(0xffffffffu, own.sdx, r); o.sdy = __shfl_down_sync(0xffffffffu, own.sdy, r);
-      o.sdz = __shfl_down_sync(0xffffffffu, own.sdz, r); o.sdw = __shfl_down_sync(0xffffffffu, own.sdw, r);
+      o.v14.x = __shfl_down_sync(0xffffffffu, own.v14.x, r); o.vdy = __shfl_down_sync(0xffffffffu, own.vdy, r);
+      o.vdz = __shfl_down_sync(0xffffffffu, own.vdz, r); o.v14.y = __shfl_down_sync(0xffffffffu, own.v14.y, r);
+      o.s14.x = __shfl_down_sync(0xffffffffu, own.s14.x, r); o.sdy = __shfl_down_sync(0xffffffffu, own.sdy, r);
+      o.sdz = __shfl_down_sync(0xffffffffu, own.sdz, r); o.s14.y = __shfl_down_sync(0xffffffffu, own.s14.y, r);
       o.vtx = __shfl_down_sync(0xffffffffu, own.vtx, r); o.vty = __shfl_down_sync(0xffffffffu, own.vty, r);
       o.xtx = __shfl_down_sync(0xffffffffu, own.xtx, r); o.xty = __shfl_down_sync(0xffffffffu, own.xty, r);
       o.T_lapl = __shfl_down_sync(0xffffffffu, own.T_lapl, r);
