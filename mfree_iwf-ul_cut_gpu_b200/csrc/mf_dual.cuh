@@ -61,7 +61,12 @@ __device__ __forceinline__ dual dlog(const dual &x) { return dchain(log(x.v), 1.
 // value is pow's and the derivative is taken as 0 (the limit of the y' term for y > 0)
 __device__ __forceinline__ dual dpow(const dual &x, const dual &y) {
   dual r = dconst(pow(x.v, y.v));
-  if (x.v > 0.) r.d = r.v * (y.d * log(x.v) + y.v * x.d / x.v);
+  if (x.v > 0.) {  // (a direction carries one parameter: most exponents and many bases have no derivative)
+    double s = 0.;
+    if (y.d != 0.) s = y.d * log(x.v);
+    if (x.d != 0.) s += y.v * x.d / x.v;
+    r.d = r.v * s;
+  }
   return r;
 }
 

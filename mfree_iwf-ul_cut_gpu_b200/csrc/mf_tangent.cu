@@ -19,8 +19,9 @@
 // product's own kernels (k_scan, k_scatter and the stable rank) run on the value positions.
 // Supported: locked grid (Green order), Brookshaw or no heat conduction, the Johnson-Cook law.
 //
-// Per step at 23,416 particles and six directions, before (one thread per particle with all six):
-// pair 974 us, force sum 281 us (one thread walking the block sums), finish 98 us, gather 82 us.
+// Per step at 23,416 particles and six directions, before (one thread per particle with all six)
+// and so: pair sums 974 / 213 us, force sum 281 us (one thread walking the block sums) / in the
+// finish kernel, finish 98 / 42 us, gather 82 / 17 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -312,9 +313,11 @@ __device__ __forceinline__ dual sum_lanes(dual x, int o) {
 
 // pair sums over the 5x5 window (interactions_gpu.cu:147-345) and the rates
 // (actions_gpu.cu:99-224), on duals: the two passes of pair_fp64_body with G lanes per particle
+// (in 64-thread blocks at 4 per SM, 214 registers and no spills: 2,991 us for the ten-step six-direction
+// pass at 23,416 particles; at 5, 168 registers and 64 B of spills, 3,148; at 8 3,046)
 constexpr int T_PAIR_BLOCK = 64;
 template <int G>
-__global__ void __launch_bounds__(T_PAIR_BLOCK, 5) k_t_pair(params P, dev_buffers D, tbuf T) {
+__global__ void __launch_bounds__(T_PAIR_BLOCK, 4) k_t_pair(params P, dev_buffers D, tbuf T) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   using R_ = pair64_rows<G>;
@@ -531,9 +534,13 @@ __device__ __noinline__ bool t_contact(const mf_tool_state &TL, const dual &qx, 
 // corrector .. invalidate (leap_frog.cu:68-92, actions_gpu.cu:135-349, tool_gpu.cu:151-221)
 // on duals, the step's tool force (report_force, output.cu:31-39; per block, then by the
 // direction's last block in block order) and the next step's cell counts
+// (The parameters are __grid_constant__: the out-of-line contact and secant functions take them by
+// reference, and copies of them in every thread's local memory wrote 100 MB a launch: 2,991 us for
+// the pass above, 2,782 without.)
 constexpr int T_FINISH_BLOCK = 128;
-__global__ void __launch_bounds__(T_FINISH_BLOCK) k_t_finish(params P, dev_buffers D, tbuf T, tparam_set TPS,
-                                                             mf_tool_state TL, int accumulate) {
+__global__ void __launch_bounds__(T_FINISH_BLOCK)
+    k_t_finish(const __grid_constant__ params P, const __grid_constant__ dev_buffers D, const __grid_constant__ tbuf T,
+               const __grid_constant__ tparam_set TPS, const __grid_constant__ mf_tool_state TL, int accumulate) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   __shared__ dual sh[4][T_FINISH_BLOCK];
