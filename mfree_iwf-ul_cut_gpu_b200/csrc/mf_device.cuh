@@ -25,7 +25,7 @@ constexpr unsigned FLAG_NONFINITE = 8u;  // pair record holds a NaN/Inf (set per
 constexpr unsigned FLAG_TOUCH = 16u;
 
 // one FP64 pair record per particle: what a neighbour j contributes to the pair sums,
-// written once per step by the predictor kernel (16 doubles = one 128-byte line)
+// written once per step by the predictor kernel (16 doubles, eight 16-byte planes in tiles: rec_word)
 enum : int {
   R_X = 0, R_Y, R_VX, R_VY, R_SXX, R_SXY, R_SYY, R_RXX, R_RXY, R_RYY, R_H, R_RHO, R_C, R_VOL, R_T, R_FLAGS,
   R_WIDTH

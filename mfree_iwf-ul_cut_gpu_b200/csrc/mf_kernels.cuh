@@ -17,10 +17,12 @@
 //                 rates: Jaumann, continuity, momentum, advection (actions_gpu.cu:99-224)
 //   k_pse         PSE heat Laplacian (interactions_gpu.cu:88-144), PSE solver only
 //   k_finish_flat corrector, friction heat, the JC elastic test, tool particles, contact,
-//                 boundary conditions, invalidation and the compensated tool-force reduction;
+//                 boundary conditions, invalidation and the compensated tool-force block sums;
 //                 with a locked grid also the next step's hashes and counts (leap_frog.cu:68-92,
 //                 actions_gpu.cu:135-162,226-349, tool_gpu.cu:151-221, output.cu:31-39)
-//   k_plastic     the JC return map of the particles the elastic test did not settle
+//   k_plastic     the JC return map of the particles the elastic test did not settle; its last block
+//                 closes the step (force of the block sums, force log, sort decision)
+//   k_close       the step's close by itself, where no material yields
 #pragma once
 
 #include "mf_device.cuh"
@@ -102,7 +104,7 @@ constexpr int PLASTIC_BLOCKS_PER_SM = 3;
 #ifndef MF_PAIR_BLOCK
 #define MF_PAIR_BLOCK 128
 #endif
-constexpr int PAIR_BLOCK = MF_PAIR_BLOCK;
+constexpr int PAIR_BLOCK = MF_PAIR_BLOCK;  // the mixed and PSE pair kernels
 // k_reorder: blocks per SM its register budget allows (REORDER_BLOCKS_PER_SM x 256 threads per
 // SM, so that a ~180k-particle grid runs in one wave)
 #ifndef REORDER_BLOCKS_PER_SM
