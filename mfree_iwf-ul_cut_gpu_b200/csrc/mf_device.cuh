@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "mf_search.h"
 #include "mfree_b200.h"
 
 namespace mf {
@@ -41,9 +42,6 @@ enum : int {
   F_WIDTH
 };
 
-// candidates a search may read past the last one (whole rounds are loaded, what lies beyond is
-// not used): the arrays of candidate records are that much longer
-constexpr int CAND_PAD = 8;
 // index of float4 word k (0..3) of particle j's FP32 pair record among N records: word 0, what the
 // distance test reads, of all particles together; the others in tiles of 32 particles, word k of a
 // tile's particles together (512 bytes), so that a warp's loads of one word are coalesced and one

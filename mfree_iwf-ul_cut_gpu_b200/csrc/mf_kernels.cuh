@@ -785,7 +785,7 @@ __device__ __forceinline__ void pair64_add(const params &P, const pair64_i &I, c
 //
 // Two passes over a particle's window. The first finds its neighbours: the G lanes test the
 // window's candidates (five contiguous ranges, ~56 particles) in FP32 on the 16-byte candidate
-// records, with a margin that keeps every pair of the exact support, STEP candidates a round, and
+// records, with a margin that keeps every pair of the exact support, CAND_STEP candidates a round, and
 // put the ones to take into lists in shared memory (two lanes fill a row from its two ends, so
 // that they share its entries evenly without counting each other's). The second takes the rows'
 // ~30 entries with the FP64 pair term, which tests the support exactly; the lanes' sums are then
@@ -793,8 +793,7 @@ __device__ __forceinline__ void pair64_add(const params &P, const pair64_i &I, c
 template <int G>
 struct pair64_rows {
   static constexpr int LANES = G > 1 ? 2 : 1;              // lanes per row
-  static constexpr int STEP = 8;                           // candidates per particle and round
-  static constexpr int U = STEP / G;                       // of which each lane's
+  static constexpr int U = CAND_STEP / G;                  // each lane's candidates of a round
   static constexpr int HALF = G == 1 ? 41 : G == 2 ? 33 : 17;  // entries per lane (rows on distinct banks)
   static constexpr int CAP = LANES * HALF;
 };
@@ -808,7 +807,7 @@ struct pair64_shared {
 template <int BS, int G>
 __device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffers &D, blk bk, unsigned *s_list) {
   using R_ = pair64_rows<G>;
-  constexpr int GROUPS = BS / G, U = R_::U, STEP = R_::STEP, LANES = R_::LANES, HALF = R_::HALF, CAP = R_::CAP;
+  constexpr int GROUPS = BS / G, U = R_::U, LANES = R_::LANES, HALF = R_::HALF, CAP = R_::CAP;
   static_assert(BS / LANES * CAP <= pair64_shared<BS>::WORDS, "lists fit");
   const int sub = (int)threadIdx.x & (G - 1), grp = (int)threadIdx.x / G;
   const int side = (int)threadIdx.x & (LANES - 1);
@@ -888,7 +887,7 @@ __device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffer
     const int j0 = n0, j1 = n1;
     if (c < 4) bounds(c + 1, n0, n1);  // the next column's bounds, in flight during this one
     const float ox = fmaf((float)(2 - c), dxc, xi);
-    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb += STEP) {
+    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb = next_round(jb, N)) {
       if (__any_sync(0xffffffffu, cnt > HALF - U)) drain();
       float4 b[U];
 #pragma unroll

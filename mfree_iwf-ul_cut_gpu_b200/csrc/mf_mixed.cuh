@@ -426,10 +426,10 @@ __device__ __forceinline__ void row_drain_parts(const rec_global &R, const unsig
 // ~28 pair terms together instead of each column's separately. Called by whole warps; `on`: the
 // particle takes part.
 template <int G, int T>
-__device__ __forceinline__ void mixed_window(const dev_buffers &D, const rec_global &R, int sub, unsigned *row,
+__device__ __forceinline__ void mixed_window(const dev_buffers &D, const rec_global &R, int N, int sub, unsigned *row,
                                              bool on, const mixed_i &I, const mixed_const &K, const geom &g, int gi,
                                              int gj, float dxc, mixed_acc &acc) {
-  constexpr int STEP = 8, U = STEP / G;
+  constexpr int U = CAND_STEP / G;
   static_assert(G == T || G == 1, "a lane per part, or one lane");
   const int low_j = gj - 2 < 0 ? 0 : gj - 2;
   const int high_j = gj + 3 > g.ny ? g.ny : gj + 3;
@@ -453,8 +453,8 @@ __device__ __forceinline__ void mixed_window(const dev_buffers &D, const rec_glo
     if (c < 4) bounds(c + 1, n0, n1);  // the next column's bounds, in flight during this one
     const float dcol = (float)(2 - c);
     const unsigned tag = (unsigned)(5 - c) << ROW_INDEX_BITS;
-    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb += STEP) {
-      if (__any_sync(0xffffffffu, cnt > mixed_rows<G>::CAP - STEP)) drain(false);
+    for (int jb = j0; __any_sync(0xffffffffu, jb < j1); jb = next_round(jb, N)) {
+      if (__any_sync(0xffffffffu, cnt > mixed_rows<G>::CAP - CAND_STEP)) drain(false);
       float4 b[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -571,7 +571,7 @@ __device__ __forceinline__ void pair_mixed_body(const params &P, const dev_buffe
     __syncwarp();
   }
   if (!LIST || __any_sync(0xffffffffu, window))
-    mixed_window<G, T>(D, R, sub, row, window, I, K, g, gi, gj, dxc, acc);
+    mixed_window<G, T>(D, R, P.N, sub, row, window, I, K, g, gi, gj, dxc, acc);
   if (LIST && sorting) build_list<G>(D, R, qc, sub, act && !I.nonfinite, I, g, gi, gj, dxc, P.skin);
   if (G > 1) {  // the lanes' parts, added up in order by the particle's first lane
     const mixed_acc own = acc;

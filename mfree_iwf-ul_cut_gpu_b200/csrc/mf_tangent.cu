@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(T_PAIR_BLOCK, 4) k_t_pair(params P, dev_buffer
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   using R_ = pair64_rows<G>;
-  constexpr int GROUPS = T_PAIR_BLOCK / G, U = R_::U, STEP = R_::STEP, LANES = R_::LANES, HALF = R_::HALF,
+  constexpr int GROUPS = T_PAIR_BLOCK / G, U = R_::U, LANES = R_::LANES, HALF = R_::HALF,
                 CAP = R_::CAP;
   __shared__ unsigned s_list[T_PAIR_BLOCK / LANES * CAP];
   const int N = P.N, dir = blockIdx.y;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(T_PAIR_BLOCK, 4) k_t_pair(params P, dev_buffer
           ++cnt;
         }
       }
-      jb += STEP;
+      jb = next_round(jb, N);
       more = __any_sync(0xffffffffu, c < 5) && !__any_sync(0xffffffffu, cnt > HALF - U);
     }
     if (LANES > 1) __syncwarp();
