@@ -1276,10 +1276,10 @@ __device__ __forceinline__ void finish_particle_phased(const params &P, const de
   B.S[q] = S;
   B.rho[q] = rho;
   B.T[q] = T;
-  // (a tool particle leaves the normal at its array position as it is: it keeps the mark of it)
-  unsigned fn = f;
-  if (P.has_tool && tool) fn = f | (f_here & FLAG_TOUCH);
-  else if (P.has_tool) fn = in_contact ? f | FLAG_TOUCH : f & ~FLAG_TOUCH;
+  // (a tool particle, and every particle while there is no tool, leaves the normal at its array
+  // position as it is, and takes the mark of it)
+  unsigned fn = f | (f_here & FLAG_TOUCH);
+  if (P.has_tool && !tool) fn = in_contact ? f | FLAG_TOUCH : f & ~FLAG_TOUCH;
   if (invalid) {  // invalidate (actions_gpu.cu:317-349)
     fn |= FLAG_BLANKED;
     newly_blanked += 1u;
