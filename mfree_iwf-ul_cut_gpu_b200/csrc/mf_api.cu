@@ -753,14 +753,18 @@ int mf_get_field(mf_ctx *ctx, int field, void *host) {
 }  // extern "C"
 
 namespace {
-// a host write of the contact forces or normals: every particle is marked as holding some
-__global__ void k_mark_touch(int N, unsigned *flags) {
+// a host write of the contact forces or normals: every particle is marked as holding some, between
+// stages in both sets (the finish kernel looks for the normal at a place by the mark in the start set)
+__global__ void k_mark_touch(int N, unsigned *flags, unsigned *start_flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) flags[i] |= FLAG_TOUCH;
+  if (i >= N) return;
+  flags[i] |= FLAG_TOUCH;
+  if (start_flags) start_flags[i] |= FLAG_TOUCH;
 }
 bool touch_field(int f) { return f == MF_FIELD_FC || f == MF_FIELD_FT || f == MF_FIELD_N; }
 cudaError_t mark_touch(mf_ctx *ctx, cudaStream_t st) {
-  k_mark_touch<<<(ctx->N + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(ctx->N, ctx->set[view_set(ctx)].flags);
+  k_mark_touch<<<(ctx->N + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(ctx->N, ctx->set[view_set(ctx)].flags,
+                                                              ctx->mid_step ? ctx->set[ctx->cur].flags : nullptr);
   return cudaGetLastError();
 }
 }  // namespace

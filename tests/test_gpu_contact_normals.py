@@ -50,3 +50,31 @@ def test_tool_removed_and_set_again(mf, grid_kind, precision):
             c.tool_set(st["tool"])
         both((k, "tool again"))
     assert left > 20, left
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("stage", [1, 2])
+def test_normals_written_between_stages(mf, stage, device):
+    torch = pytest.importorskip("torch")
+    st = scene(mf)
+    a, b = load(mf, st, 0, 0), load(mf, st, 0, 0)
+    rng = np.random.default_rng(7)
+    n = rng.normal(0.0, 1.0, (st["N"], 2))
+    on_device = torch.from_numpy(n).cuda()
+    b.set("n", b.get("n"))
+    for k in range(4):
+        for c in (a, b):
+            c.stage(k)
+            if k == stage and device:
+                c.set_device("n", on_device.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            elif k == stage:
+                c.set("n", n)
+    for k in range(3):
+        for f in FIELDS:
+            assert bits_equal(a.get(f), b.get(f)), (k, f)
+        wp = a.get("tool_p") == 0.0
+        out = wp & (np.abs(a.get("fc")).sum(axis=1) == 0) & (a.get("fixed") == 0.0)
+        assert not a.get("n")[out].any()  # outside the tool: no normal
+        b.set("n", b.get("n"))
+        for c in (a, b):
+            c.step(1)
