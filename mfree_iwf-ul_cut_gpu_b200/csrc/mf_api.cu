@@ -249,12 +249,6 @@ bool list_mode(const mf_ctx *ctx) {
 }
 
 void set_list_mode(mf_ctx *ctx) {
-  // the EOS sound speed of every particle: the device's float rounding of the same IEEE
-  // operations, computed once
-  ctx->P.eos_c0 = (double)sqrtf((float)(ctx->P.phys.K / ctx->P.phys.rho0));
-  ctx->P.inv_wdeltap = 1. / ctx->P.corr.wdeltap;
-  ctx->P.alpha_half = 0.5 * ctx->P.corr.alpha;
-  ctx->P.eta2 = ctx->P.corr.eta * ctx->P.corr.eta;
   ctx->P.verlet = list_mode(ctx) ? 1 : 0;
   ctx->P.fuse = ctx->P.verlet && (ctx->flags & MF_OPT_FUSED_PREDICTOR) ? 1 : 0;
   // at most half a cell: the lists are built over the 7x7 cells around a particle, which hold
@@ -911,6 +905,13 @@ int mf_set_constants(mf_ctx *ctx, const mf_phys_constants *phys, const mf_corr_c
   params &P = ctx->P;
   P.phys = *phys;
   P.corr = *corr;
+  // what the kernels need of them in another form (here, where they are set: a batch or the
+  // differentiable step may be the next to use them); the EOS sound speed of every particle with the
+  // device's float rounding of the same IEEE operations
+  P.eos_c0 = (double)sqrtf((float)(P.phys.K / P.phys.rho0));
+  P.inv_wdeltap = 1. / P.corr.wdeltap;
+  P.alpha_half = 0.5 * P.corr.alpha;
+  P.eta2 = P.corr.eta * P.corr.eta;
   P.plastic = joco ? 1 : 0;
   if (joco) P.joco = *joco;
   else std::memset(&P.joco, 0, sizeof(P.joco));

@@ -787,10 +787,6 @@ int run_mean_force(const params &P_in, const dev_buffers &C, const state_set &no
   params P = P_in;
   P.staged = 0;
   P.verlet = 0;
-  P.inv_wdeltap = 1. / P.corr.wdeltap;
-  P.alpha_half = 0.5 * P.corr.alpha;
-  P.eta2 = P.corr.eta * P.corr.eta;
-  P.eos_c0 = (double)sqrtf((float)(P.phys.K / P.phys.rho0));
   const int N = P.N, nd = std::max(1, n_directions);
   const int scan_tiles = (max_cell + SCAN_TILE - 1) / SCAN_TILE + 1;
   const int nf = (N + T_FINISH_BLOCK - 1) / T_FINISH_BLOCK;
