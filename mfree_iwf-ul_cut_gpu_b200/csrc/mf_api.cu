@@ -1283,6 +1283,8 @@ int batch_build_fused(mf_batch *b, int K) {
 // one parent graph: a child graph of K steps per context, no edges between them (or, where
 // the systems allow it, the batched kernels)
 int batch_build(mf_batch *b, int K) {
+  b->fused = batch_can_fuse(b);  // (decided anew: the contexts' options may have changed)
+  if (!b->fused) b->form = MF_BATCH_PHASES;
   if (b->fused) return batch_build_fused(b, K);
   batch_release(b);
   cudaGraph_t parent = nullptr;
@@ -1457,7 +1459,7 @@ int mf_batch_set_form(mf_batch *b, int form, int blocks_per_sm, int steps_per_la
       (steps_per_launch & 1))
     return MF_ERR_INVALID;
   // child-graph batches have no phases; the persistent kernel steps the mixed form only
-  if (form == MF_BATCH_PERSISTENT && (!b->fused || b->ctx[0]->P.precision != MF_PRECISION_MIXED))
+  if (form == MF_BATCH_PERSISTENT && (!batch_can_fuse(b) || b->ctx[0]->P.precision != MF_PRECISION_MIXED))
     return MF_ERR_INVALID;
   if (cudaSetDevice(b->device) != cudaSuccess || cudaStreamSynchronize(b->stream) != cudaSuccess) return MF_ERR_CUDA;
   b->form = form;

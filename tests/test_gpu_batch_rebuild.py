@@ -33,3 +33,31 @@ def test_constants_changed(mf, precision):
     for x, y in zip(batched, single):
         assert_same(x, y)
     b.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_one_instance_changes_precision(mf, precision):
+    sts, (batched, single) = two_sets(mf, precision)
+    b = mf.Batch(batched, steps_per_launch=4)
+    b.step(1)
+    for c in single:
+        c.step(4)
+    for c in (batched[1], single[1]):
+        c.set_options(mf.THERMAL_BROOKSHAW, mf.JC_JOHNSON_COOK, 1 - precision)
+    b.set_form(mf.BATCH_PHASES, steps_per_launch=4)
+    assert not b.fused  # the batched kernels serve one precision
+    b.step(1)
+    for c in single:
+        c.step(4)
+    for x, y in zip(batched, single):
+        assert_same(x, y)
+    for c in (batched[1], single[1]):
+        c.set_options(mf.THERMAL_BROOKSHAW, mf.JC_JOHNSON_COOK, precision)
+    b.set_form(mf.BATCH_PHASES, steps_per_launch=4)
+    assert b.fused
+    b.step(1)
+    for c in single:
+        c.step(4)
+    for x, y in zip(batched, single):
+        assert_same(x, y)
+    b.close()
