@@ -393,6 +393,12 @@ __device__ __forceinline__ double2 rec_plane(const double *__restrict__ rec, int
 // distance (a NaN or Inf in the record, a position the FP32 offset cannot hold, a density outside
 // float's range) at NaN, which every test takes.
 constexpr unsigned CAND_TOOL = 0x80000000u, CAND_ANY = 0x40000000u, CAND_COLUMN = 0x3fffffffu;
+// The record holds the cell's row as a float and its column in 30 bits. On a grid with more rows or
+// columns than these count, every particle is taken whatever its distance, and its cell comes from
+// its hash.
+__device__ __forceinline__ bool cand_counts_cells(const geom &g) {
+  return g.ny <= (1 << 24) && g.nx <= (int)CAND_COLUMN + 1;
+}
 __host__ __device__ __forceinline__ size_t rec_doubles(int N) { return (size_t)((N + 31) / 32) * 32 * R_WIDTH; }
 __device__ __forceinline__ const float4 *rec_cand(const double *rec, int N) {
   return reinterpret_cast<const float4 *>(rec + rec_doubles(N));
@@ -492,11 +498,11 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
     const geom g = *D.g;
     const int ci = hsh / g.ny, cj = hsh - ci * g.ny;
     const double rx = pos.x - (g.bbmin_x + ci * g.dx), ry = pos.y - (g.bbmin_y + cj * g.dx);
-    const bool any = (rf & FLAG_NONFINITE) || !(fabs(rx) <= 4. * g.dx && fabs(ry) <= 4. * g.dx) ||
+    const bool any = (rf & FLAG_NONFINITE) || !cand_counts_cells(g) || !(fabs(rx) <= 4. * g.dx && fabs(ry) <= 4. * g.dx) ||
                      !(fabs(rho) >= 1e-30 && fabs(rho) <= 1e30) || !(h >= 1e-15 && h <= 1e15);
     const_cast<float4 *>(rec_cand(D.rec, P.N))[q] =
         make_float4(blanked ? __int_as_float(0x7f800000) : any ? __int_as_float(0x7fffffff) : (float)rx, (float)ry,
-                    __uint_as_float((unsigned)ci | (tool ? CAND_TOOL : 0u) | (any ? CAND_ANY : 0u)), (float)cj);
+                    __uint_as_float(((unsigned)ci & CAND_COLUMN) | (tool ? CAND_TOOL : 0u) | (any ? CAND_ANY : 0u)), (float)cj);
     const float fv[12] = {(float)vel.x, (float)vel.y, (float)sxx, (float)sxy, (float)syy, (float)Rxx,
                           (float)Rxy, (float)Ryy, (float)h, (float)rho, (float)c, (float)vol};
 #pragma unroll
@@ -872,7 +878,12 @@ __device__ __forceinline__ void pair_fp64_body(const params &P, const dev_buffer
     cnt = 0;
     if (LANES > 1) __syncwarp();
   };
-  const int gi = (int)(marks & CAND_COLUMN), gj = (int)ci.w;
+  int gi = (int)(marks & CAND_COLUMN), gj = (int)ci.w;
+  if (!cand_counts_cells(g)) {
+    const int c = D.hash_cur[qc];
+    gi = c / g.ny;
+    gj = c - gi * g.ny;
+  }
   const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
   auto bounds = [&](int c, int &j0, int &j1) {  // window column c's particles
     const int ii = gi - 2 + c;

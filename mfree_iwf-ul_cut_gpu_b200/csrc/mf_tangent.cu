@@ -225,10 +225,10 @@ __global__ void __launch_bounds__(128) k_t_reorder(params P, dev_buffers D, tbuf
   const geom g = *D.g;
   const int ci = u.y / g.ny, cj = u.y - ci * g.ny;
   const double rx = pos[0].v - (g.bbmin_x + ci * g.dx), ry = pos[1].v - (g.bbmin_y + cj * g.dx);
-  const bool any = !(fabs(rx) <= 4. * g.dx && fabs(ry) <= 4. * g.dx) ||
+  const bool any = !cand_counts_cells(g) || !(fabs(rx) <= 4. * g.dx && fabs(ry) <= 4. * g.dx) ||
                    !(fabs(rho.v) >= 1e-30 && fabs(rho.v) <= 1e30) || !(h >= 1e-15 && h <= 1e15);
   T.cand[q] = make_float4(blanked ? __int_as_float(0x7f800000) : any ? __int_as_float(0x7fffffff) : (float)rx, (float)ry,
-                          __uint_as_float((unsigned)ci | (tool ? CAND_TOOL : 0u) | (any ? CAND_ANY : 0u)), (float)cj);
+                          __uint_as_float(((unsigned)ci & CAND_COLUMN) | (tool ? CAND_TOOL : 0u) | (any ? CAND_ANY : 0u)), (float)cj);
 }
 
 // 1 / x on duals (rcp64 unless the value may lie outside float's range)
@@ -341,7 +341,12 @@ __global__ void __launch_bounds__(T_PAIR_BLOCK, 4) k_t_pair(params P, dev_buffer
   const float Rf = 2.00001f * (float)hf.v + 1e-5f * dxc;  // as in pair_fp64_body
   const float R2 = Rf * Rf;
   const float xi = any_i ? __int_as_float(0x7fffffff) : ci.x;
-  const int gi = (int)(marks & CAND_COLUMN), gj = (int)ci.w;
+  int gi = (int)(marks & CAND_COLUMN), gj = (int)ci.w;
+  if (!cand_counts_cells(g)) {
+    const int c = D.hash_cur[qc];
+    gi = c / g.ny;
+    gj = c - gi * g.ny;
+  }
   const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
   tpair_i I;
   I.tool = fi & FLAG_TOOL;
