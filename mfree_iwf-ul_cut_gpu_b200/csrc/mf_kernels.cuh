@@ -772,10 +772,11 @@ __device__ __forceinline__ void pair64_add(const params &P, const pair64_i &I, c
       irho = 1. / rs;
       iden = 1. / den;
     }
-    // Monaghan viscosity for approaching pairs
+    // Monaghan viscosity for approaching pairs (outside the support, where W = 0, left out: without
+    // eta the denominator of nearly coincident particles is outside float's range)
     const double nmu = __dmul_rn(__dmul_rn(hij, nvr), iden);
     const double ac = __dmul_rn(P.alpha_half, __dadd_rn(I.c, r[6].x));
-    const double pi = nvr > 0. ? __dmul_rn(__dmul_rn(fma(P.corr.beta, nmu, ac), nmu), irho) : 0.;
+    const double pi = nvr > 0. && (in_support || careful) ? __dmul_rn(__dmul_rn(fma(P.corr.beta, nmu, ac), nmu), irho) : 0.;
     a.vt[0] = fma(pi, wx, a.vt[0]);
     a.vt[1] = fma(pi, wy, a.vt[1]);
     const double xs = __dmul_rn(w, irho);
