@@ -158,6 +158,21 @@ __device__ __forceinline__ void cubic_spline_fp64(double xij, double yij, double
 }
 
 // ---------------------------------------------------------------------------------------
+// 1 / x for 1e-37 <= |x| <= 1e37 (x and 1 / x normal floats: the approximation below takes and gives
+// zero for subnormal ones) by one third-order Newton step from the FP32 reciprocal approximation y of
+// xf, x rounded to float: the residual r, with that rounding below 1.8e-7, cubed is below 6e-21, and
+// y (1 + r + r^2) is rounded once, so the result is within 0.5001 units in the last place of 1 / x, in
+// three multiply-adds.
+__device__ __forceinline__ double rcp64_from(double x, float xf) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(xf));
+  const double y0 = (double)y;
+  const double r = fma(-x, y0, 1.);
+  return fma(y0, fma(r, r, r), y0);
+}
+__device__ __forceinline__ double rcp64(double x) { return rcp64_from(x, (float)x); }
+
+// ---------------------------------------------------------------------------------------
 // artificial stress (actions_gpu.cu:35-39, 53-97)
 __device__ __forceinline__ void artificial_stress(double rhoi, double pi, double Sx, double Sy, double Sz,
                                                   double eps, double &Rxx, double &Rxy, double &Ryy) {

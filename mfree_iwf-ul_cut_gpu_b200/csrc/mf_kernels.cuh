@@ -692,18 +692,6 @@ static __global__ void __launch_bounds__(BLOCK, REORDER_BLOCKS_PER_SM) k_reorder
 // visiting the columns in x order and each range in array order is the reference's
 // neighbour order (x-cell outer, y-cell inner, sorted order within a cell).
 
-// 1 / x for x within float's range by one third-order Newton step from the FP32 reciprocal
-// approximation y of x: its relative error, with x's rounding to float below 2e-7, cubed is below
-// 1e-20, so the result is rounded like a division to within the last bit, in three multiply-adds.
-__device__ __forceinline__ double rcp64_from(double x, float xf) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(xf));
-  const double y0 = (double)y;
-  const double r = fma(-x, y0, 1.);
-  return fma(y0, fma(r, r, r), y0);
-}
-__device__ __forceinline__ double rcp64(double x) { return rcp64_from(x, (float)x); }
-
 // the i particle's values of the FP64 pair sums
 struct pair64_i {
   double x, y, vx, vy, sxx, sxy, syy, Rxx, Rxy, Ryy, h, rho, c, T;
