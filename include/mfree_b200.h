@@ -422,10 +422,10 @@ int mf_batch_destroy(mf_batch *batch);
    the window of the tool force (report_force, output.cu:31-39: [0] cutting Fc, [1] feed Ff)
    and, for param 0..5 = Johnson-Cook A, B, n, C, m or the friction coefficient mu, its
    derivative with respect to that parameter (forward-mode tangents through every step; param
-   -1: the mean only). The context's state is not changed; the work memory (about 1.2 KB per
-   particle and direction) stays with the context until its particles are created again or it is
-   destroyed. Locked Green grid, Brookshaw or no
-   conduction, Johnson-Cook law only (MF_ERR_INVALID otherwise). ---- */
+   -1: the mean only). The context's state is not changed. Work memory is about 1.2 KB per particle
+   and direction; up to 1 GiB of it stays with the context until its particles are created again
+   or it is destroyed, more is given back before the call returns. Locked Green grid, Brookshaw or
+   no conduction, Johnson-Cook law only (MF_ERR_INVALID otherwise). ---- */
 int mf_tangent_mean_force(mf_ctx *ctx, int skip_steps, int window_steps, int param, double out_mean[2],
                           double out_dmean[2]);
 /* the same for all six parameters in one pass (six tangent directions carried together):

@@ -778,6 +778,10 @@ cudaError_t launch(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, int
 // direction and one with six add each direction up alike
 constexpr int lanes(int N) { return N <= 8192 ? 4 : N <= 18944 ? 2 : 1; }
 
+// Work memory kept for a context's next call; a larger one is given back, so that contexts with many
+// particles do not hold several GB each while they step.
+constexpr size_t KEEP_BYTES = (size_t)1 << 30;
+
 }  // namespace
 
 void release(workspace &ws) {
@@ -877,6 +881,7 @@ int run_mean_force(const params &P_in, const dev_buffers &C, const state_set &no
   if (e == cudaSuccess) e = cudaMemcpyAsync(&st, D.st, sizeof(st), cudaMemcpyDeviceToHost, stream);
   const cudaError_t es = cudaStreamSynchronize(stream);
   if (e == cudaSuccess) e = es;
+  if (ws.bytes > KEEP_BYTES) release(ws);
   if (e != cudaSuccess) {
     *cuda_err = (int)e;
     return MF_ERR_CUDA;

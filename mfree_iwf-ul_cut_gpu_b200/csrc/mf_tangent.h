@@ -6,8 +6,9 @@
 namespace mf {
 namespace tg {
 
-// Device memory of the differentiable step, kept by the context between calls (its size follows
-// the particle count and the number of directions) and freed with the context's particles.
+// Device memory of the differentiable step (its size follows the particle count and the number of
+// directions): up to KEEP_BYTES of it kept by the context between calls and freed with the context's
+// particles, more only during a call.
 struct workspace {
   void *mem = nullptr;
   size_t bytes = 0;
