@@ -301,10 +301,7 @@ int launch_cells(mf_ctx *ctx, bool step_mode) {
   bind_sets(ctx);
   if (!ctx->G.locked)
     TRY(launch(ctx, EARLY, k_bbox, ctx->bbox_blocks, BLOCK, N, (const double2 *)ctx->D.A.pos, (const double *)ctx->D.A.h, ctx->D));
-  if (!(step_mode && fused_step(ctx))) {
-    const int hash_blocks = std::max(nb, (ctx->scan_tiles + BLOCK - 1) / BLOCK);
-    TRY(launch(ctx, EARLY, k_hash_count, hash_blocks, BLOCK, N, ctx->D.A, ctx->D, ctx->scan_tiles));
-  }
+  if (!(step_mode && fused_step(ctx))) TRY(launch(ctx, EARLY, k_hash_count, nb, BLOCK, N, ctx->D.A, ctx->D));
   const int verlet = step_mode ? ctx->P.verlet : 0;  // a sort outside a step always sorts
   TRY(launch(ctx, EARLY, k_scan, ctx->scan_tiles, SCAN_THREADS, ctx->D, N, verlet));
   TRY(launch(ctx, EARLY, k_scatter, nb, BLOCK, N, ctx->D, verlet));
@@ -422,8 +419,7 @@ int prime_counts(mf_ctx *ctx) {
   if (!fused_step(ctx) || ctx->counts_ready) return MF_OK;
   bind_sets(ctx);
   const int nb = (ctx->N + BLOCK - 1) / BLOCK;
-  const int hash_blocks = std::max(nb, (ctx->scan_tiles + BLOCK - 1) / BLOCK);
-  k_hash_count<<<hash_blocks, BLOCK, 0, ctx->stream>>>(ctx->N, ctx->D.A, ctx->D, ctx->scan_tiles);
+  k_hash_count<<<nb, BLOCK, 0, ctx->stream>>>(ctx->N, ctx->D.A, ctx->D);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { ctx->last_cuda_err = (int)e; return MF_ERR_CUDA; }
   // with neighbour lists the next step sorts (and builds the lists): any nonzero value
@@ -1191,7 +1187,6 @@ int batch_build_fused(mf_batch *b, int K) {
       std::memset(&x, 0, sizeof(x));
       x.P = c->P;
       x.D = c->D;
-      x.scan_tiles = c->scan_tiles;
     }
     c->cur = saved;
     bind_sets(c);

@@ -12,11 +12,10 @@
 
 namespace mf {
 
-// one system's step parameters, buffers (bound to one parity of its double buffer) and scan size
+// one system's step parameters and buffers (bound to one parity of its double buffer)
 struct __align__(16) batch_entry {
   params P;
   dev_buffers D;
-  int scan_tiles;
 };
 
 // one batched launch: entries of every system and first[k] = the first grid block of system k

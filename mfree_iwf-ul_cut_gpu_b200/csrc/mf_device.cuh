@@ -130,34 +130,6 @@ constexpr int LIST_INDEX_BITS = 26;
 constexpr unsigned LIST_INDEX_MASK = (1u << LIST_INDEX_BITS) - 1u;
 
 // ---------------------------------------------------------------------------------------
-// SPH kernel function: cubic spline (kernels.cuh:30-70). hi enters through h1 = 1/hi and
-// fourh2 = 4*hi*hi, computed once per particle i exactly as the reference computes them
-// per pair. Returns false (w = 0) outside the support or for r^2 < 1e-8.
-// Also returns dwr = der*fac, the radial factor of the gradient (grad W = dwr * x_ij), which
-// is (e_ij . grad W) / r of the Brookshaw Laplacian.
-__device__ __forceinline__ void cubic_spline_fp64(double xij, double yij, double rr2, double h1,
-                                                  double &w, double &w_x, double &w_y, double &dwr) {
-  constexpr double PI_FAC = 0.454728408833987;
-  double der, val;
-  double rad = (double)sqrtf((float)rr2);
-  double q = rad * h1;
-  double fac = PI_FAC * h1 * h1;
-  if (q > 1) {
-    double _2mq = 2 - q;
-    double _2mq2 = _2mq * _2mq;
-    val = 0.25 * _2mq2 * _2mq2 * _2mq2;
-    der = -0.75 * _2mq2 * h1 / rad;
-  } else {
-    val = 1 - 1.5 * q * q * (1 - 0.5 * q);
-    der = -3.0 * q * (1 - 0.75 * q) * h1 / rad;
-  }
-  w = val * fac;
-  w_x = der * xij * fac;
-  w_y = der * yij * fac;
-  dwr = der * fac;
-}
-
-// ---------------------------------------------------------------------------------------
 // 1 / x for 1e-37 <= |x| <= 1e37 (x and 1 / x normal floats: the approximation below takes and gives
 // zero for subnormal ones) by one third-order Newton step from the FP32 reciprocal approximation y of
 // xf, x rounded to float: the residual r, with that rounding below 1.8e-7, cubed is below 6e-21, and
@@ -418,22 +390,6 @@ __device__ __forceinline__ void line_through_rn(double x1, double y1, double x2,
   vertical = 0;
   a = __ddiv_rn(__dsub_rn(__dmul_rn(y1, 1.), __dmul_rn(1., y2)), detM);
   b = __ddiv_rn(__dsub_rn(__dmul_rn(y2, x1), __dmul_rn(x2, y1)), detM);
-}
-
-__device__ __forceinline__ void tool_translate_rn(mf_tool_state &T, double dt) {
-  double sx = __dmul_rn(dt, T.vel[0]), sy = __dmul_rn(dt, T.vel[1]);
-  for (int i = 0; i < T.num_seg; ++i) {
-    mf_segment &s = T.seg[i];
-    s.left[0] = __dadd_rn(s.left[0], sx);
-    s.left[1] = __dadd_rn(s.left[1], sy);
-    s.right[0] = __dadd_rn(s.right[0], sx);
-    s.right[1] = __dadd_rn(s.right[1], sy);
-    line_through_rn(s.left[0], s.left[1], s.right[0], s.right[1], s.a, s.b, s.vertical);
-  }
-  if (T.has_fillet) {
-    T.fillet.p[0] = __dadd_rn(T.fillet.p[0], sx);
-    T.fillet.p[1] = __dadd_rn(T.fillet.p[1], sy);
-  }
 }
 
 __device__ __forceinline__ bool isnaninf(double v) { return isnan(v) || isinf(v); }

@@ -222,7 +222,7 @@ __device__ __forceinline__ int cell_coordinate(double x, const geom &g) {
 
 // ---------------------------------------------------------------------------------------
 // cell hash + count (compute_hashes, grid.cu:34-51)
-static __global__ void __launch_bounds__(BLOCK) k_hash_count(int N, state_set A, dev_buffers D, int num_scan_tiles) {
+static __global__ void __launch_bounds__(BLOCK) k_hash_count(int N, state_set A, dev_buffers D) {
   MF_PDL_WAIT();
   MF_PDL_TRIGGER();
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -593,7 +593,7 @@ static __device__ __noinline__ void tool_advance_warp(const mf_tool_state *prev,
   }
 }
 
-// the step's tool (written by the pair kernel) into shared memory, copied word by word by the
+// the step's tool (written by the reorder kernel) into shared memory, copied word by word by the
 // block's threads
 __device__ __forceinline__ void tool_load_shared(mf_tool_state &T, const dev_buffers &D) {
   constexpr int WORDS = (int)(sizeof(mf_tool_state) / sizeof(double));
