@@ -185,9 +185,7 @@ def vtk_tools(R):
     R.refh_tool_update.argtypes = [C.c_double]
     out = {}
     cwd = os.getcwd()
-    scratch = ROOT / "_work"
-    scratch.mkdir(exist_ok=True)
-    with tempfile.TemporaryDirectory(dir=scratch) as d:
+    with tempfile.TemporaryDirectory() as d:
         os.chdir(d)
         try:
             os.mkdir("results")
@@ -218,9 +216,7 @@ def vtk_particles(R, rng, n=400):
          "fixed": (rng.random(n) < 0.1).astype(float), "tool_p": (rng.random(n) < 0.2).astype(float)}
     R.refh_vtk_particles.argtypes = [C.c_int, C.c_int] + [C.c_void_p] * 10
     cwd = os.getcwd()
-    scratch = ROOT / "_work"
-    scratch.mkdir(exist_ok=True)
-    with tempfile.TemporaryDirectory(dir=scratch) as tdir:
+    with tempfile.TemporaryDirectory() as tdir:
         os.chdir(tdir)
         try:
             os.mkdir("results")
