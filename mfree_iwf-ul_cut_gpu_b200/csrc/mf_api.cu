@@ -1102,8 +1102,8 @@ struct mf_batch {
   bool fused = false;
   int pair_bs = PAIR_BLOCK;          // block size of the batched pair kernel (tuned)
   batch_entry *d_entries = nullptr;  // [2][n]: every system bound to each parity of its buffers
-  int *d_first = nullptr;            // 4 maps of n + 1 first blocks: scan, 256-thread phases, pair, plastic
-  int grid[4] = {0, 0, 0, 0};
+  int *d_first = nullptr;            // NUM_MAPS maps of n + 1 first blocks
+  int grid[NUM_MAPS] = {};
   // MF_BATCH_PERSISTENT: K steps in one cooperative launch of persist_bps blocks per SM
   int form = MF_BATCH_PHASES;
   int persist_bps = 0;           // 0: as many as are resident
@@ -1150,13 +1150,13 @@ int batch_kernel(mf_batch *b, void (*kernel)(KArgs...), int grid, int block, Arg
 
 // the pair phase (and PSE) of one step at the tuned block size
 template <int BS>
-int batch_pair(mf_batch *b, const params &P0, batch_map m) {
+int batch_pair(mf_batch *b, const params &P0, batch_map m, batch_map m_pse) {
   const bool mixed = P0.precision == MF_PRECISION_MIXED;
-  if (mixed) TRY(batch_kernel(b, kb_pair_mixed<BS>, b->grid[2], BS, m));
-  else TRY(batch_kernel(b, kb_pair_fp64<BS>, b->grid[2], BS, m));
+  if (mixed) TRY(batch_kernel(b, kb_pair_mixed<BS>, b->grid[MAP_PAIR], BS, m));
+  else TRY(batch_kernel(b, kb_pair_fp64<BS>, b->grid[MAP_PAIR], BS, m));
   if (P0.thermal_solver == MF_THERMAL_PSE && P0.thermal_wp) {
-    if (mixed) TRY(batch_kernel(b, kb_pse_mixed<BS>, b->grid[2], BS, m));
-    else TRY(batch_kernel(b, kb_pse<BS>, b->grid[2], BS, m));
+    if (mixed) TRY(batch_kernel(b, kb_pse_mixed<BS>, b->grid[MAP_PSE], BS, m_pse));
+    else TRY(batch_kernel(b, kb_pse<BS>, b->grid[MAP_PSE], BS, m_pse));
   }
   return MF_OK;
 }
@@ -1170,7 +1170,7 @@ int batch_build_fused(mf_batch *b, int K) {
   batch_release(b);
   const int n = (int)b->ctx.size();
   std::vector<batch_entry> e(2 * (size_t)n);
-  std::vector<int> first(4 * (size_t)(n + 1), 0);
+  std::vector<int> first(NUM_MAPS * (size_t)(n + 1), 0);
   long long total_n = 0;
   for (mf_ctx *c : b->ctx) total_n += c->N;
   const int sms = b->ctx[0]->sm_count;
@@ -1191,13 +1191,18 @@ int batch_build_fused(mf_batch *b, int K) {
     c->cur = saved;
     bind_sets(c);
     const int pair_bs = b->form == MF_BATCH_PERSISTENT ? PERSIST_BLOCK : b->pair_bs;
-    // particles per pair block
-    const int per = pair_bs / (c->P.precision == MF_PRECISION_MIXED ? 1 : pair64_lanes(c->N));
-    const int blocks[4] = {c->scan_tiles, (c->N + BLOCK - 1) / BLOCK, (c->N + per - 1) / per,
-                           c->P.plastic ? 1 + (int)std::max<long long>(1, (long long)sms * PLASTIC_BLOCKS_PER_SM * c->N / total_n) : 1};
-    for (int m = 0; m < 4; ++m) first[(size_t)m * (n + 1) + k + 1] = first[(size_t)m * (n + 1) + k] + blocks[m];
+    // particles per pair block and PSE block (the mixed pair sums run at one lane in a batch, the heat
+    // at the system's own lanes)
+    const bool mixed = c->P.precision == MF_PRECISION_MIXED;
+    const int per = pair_bs / (mixed ? 1 : pair64_lanes(c->N));
+    const int per_pse = pair_bs / (mixed ? mixed_parts(c->N) : pair64_lanes(c->N));
+    const int blocks[NUM_MAPS] = {
+        c->scan_tiles, (c->N + BLOCK - 1) / BLOCK, (c->N + per - 1) / per,
+        c->P.plastic ? 1 + (int)std::max<long long>(1, (long long)sms * PLASTIC_BLOCKS_PER_SM * c->N / total_n) : 1,
+        (c->N + per_pse - 1) / per_pse};
+    for (int m = 0; m < NUM_MAPS; ++m) first[(size_t)m * (n + 1) + k + 1] = first[(size_t)m * (n + 1) + k] + blocks[m];
   }
-  for (int m = 0; m < 4; ++m) b->grid[m] = first[(size_t)m * (n + 1) + n];
+  for (int m = 0; m < NUM_MAPS; ++m) b->grid[m] = first[(size_t)m * (n + 1) + n];
   if (!b->d_entries) {
     if (cudaMalloc(&b->d_entries, sizeof(batch_entry) * e.size()) != cudaSuccess) return MF_ERR_NOMEM;
     if (cudaMalloc(&b->d_first, sizeof(int) * first.size()) != cudaSuccess) return MF_ERR_NOMEM;
@@ -1225,7 +1230,7 @@ int batch_build_fused(mf_batch *b, int K) {
     A.first = b->d_first;
     A.n = n;
     A.K = K;
-    for (int m = 0; m < 4; ++m) A.grid[m] = b->grid[m];
+    for (int m = 0; m < NUM_MAPS; ++m) A.grid[m] = b->grid[m];
     A.pse = P0.thermal_solver == MF_THERMAL_PSE && P0.thermal_wp ? 1 : 0;
     A.plastic = P0.plastic ? 1 : 0;
     A.paired = P0.jc_model == MF_JC_TANH ? 0 : 1;
@@ -1241,25 +1246,25 @@ int batch_build_fused(mf_batch *b, int K) {
   }
   for (int st = 0; st < K && rc == MF_OK && b->form != MF_BATCH_PERSISTENT; ++st) {
     const batch_entry *ent = b->d_entries + (size_t)(st & 1) * n;
-    const batch_map m_scan{ent, b->d_first, n}, m_256{ent, b->d_first + (n + 1), n},
-        m_pair{ent, b->d_first + 2 * (n + 1), n}, m_pl{ent, b->d_first + 3 * (n + 1), n};
-    rc = batch_kernel(b, kb_scan, b->grid[0], SCAN_THREADS, m_scan);
-    if (rc == MF_OK) rc = batch_kernel(b, kb_scatter, b->grid[1], BLOCK, m_256);
-    if (rc == MF_OK) rc = mixed ? batch_kernel(b, kb_reorder<true>, b->grid[1], BLOCK, m_256)
-                                : batch_kernel(b, kb_reorder<false>, b->grid[1], BLOCK, m_256);
+    auto map = [&](int m) { return batch_map{ent, b->d_first + m * (n + 1), n}; };
+    const batch_map m_scan = map(MAP_SCAN), m_256 = map(MAP_256), m_pl = map(MAP_PLASTIC);
+    rc = batch_kernel(b, kb_scan, b->grid[MAP_SCAN], SCAN_THREADS, m_scan);
+    if (rc == MF_OK) rc = batch_kernel(b, kb_scatter, b->grid[MAP_256], BLOCK, m_256);
+    if (rc == MF_OK) rc = mixed ? batch_kernel(b, kb_reorder<true>, b->grid[MAP_256], BLOCK, m_256)
+                                : batch_kernel(b, kb_reorder<false>, b->grid[MAP_256], BLOCK, m_256);
     if (rc == MF_OK) {
       switch (b->pair_bs) {
-        case 64: rc = batch_pair<64>(b, P0, m_pair); break;
-        case 256: rc = batch_pair<256>(b, P0, m_pair); break;
-        default: rc = batch_pair<128>(b, P0, m_pair); break;
+        case 64: rc = batch_pair<64>(b, P0, map(MAP_PAIR), map(MAP_PSE)); break;
+        case 256: rc = batch_pair<256>(b, P0, map(MAP_PAIR), map(MAP_PSE)); break;
+        default: rc = batch_pair<128>(b, P0, map(MAP_PAIR), map(MAP_PSE)); break;
       }
     }
-    if (rc == MF_OK) rc = batch_kernel(b, kb_finish, b->grid[1], FINISH_BLOCK, m_256);
+    if (rc == MF_OK) rc = batch_kernel(b, kb_finish, b->grid[MAP_256], FINISH_BLOCK, m_256);
     if (rc == MF_OK && P0.plastic)
-      rc = P0.jc_model == MF_JC_TANH ? batch_kernel(b, kb_plastic<false>, b->grid[3], BLOCK, m_pl)
-                                     : batch_kernel(b, kb_plastic<true>, b->grid[3], BLOCK, m_pl);
+      rc = P0.jc_model == MF_JC_TANH ? batch_kernel(b, kb_plastic<false>, b->grid[MAP_PLASTIC], BLOCK, m_pl)
+                                     : batch_kernel(b, kb_plastic<true>, b->grid[MAP_PLASTIC], BLOCK, m_pl);
     else if (rc == MF_OK)
-      rc = batch_kernel(b, kb_close, b->grid[3], BLOCK, m_pl);
+      rc = batch_kernel(b, kb_close, b->grid[MAP_PLASTIC], BLOCK, m_pl);
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(b->stream, &g);

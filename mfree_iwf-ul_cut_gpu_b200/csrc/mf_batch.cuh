@@ -18,6 +18,9 @@ struct __align__(16) batch_entry {
   dev_buffers D;
 };
 
+// the batch's block maps: cell scan, phases of 256 threads per block, pair sums, return map, PSE heat
+enum : int { MAP_SCAN = 0, MAP_256, MAP_PAIR, MAP_PLASTIC, MAP_PSE, NUM_MAPS };
+
 // one batched launch: entries of every system and first[k] = the first grid block of system k
 // (n + 1 values, first[n] = the grid size)
 struct batch_map {

@@ -989,62 +989,60 @@ static __global__ void __launch_bounds__(PAIR64_BLOCK, 8) k_pair_fp64(params P, 
 // PSE heat Laplacian (interactions_gpu.cu:88-144): every particle of the window, blanked
 // ones included; alpha taken through the reference's half-length texture binding (:405).
 // G lanes per particle (pair64_lanes, as in the pair kernel) take a column's candidates in turn, U
-// at a time with all their loads in flight, and their sums are added in a fixed tree; a block takes
-// BS / G particles at a time until its system's are done. The reference's sqrt, its two divisions by
-// h^2 and its division by rho_j are gone from the pair: r^2 is not rooted and squared again, 1 / h^2
-// and the Gaussian's factor are the particle's, m / rho_j is in the record. Pair stage with it at
-// 23,416 particles: 60.4 us before (this kernel 39.8, one thread per particle), 33.8 so.
+// at a time with all their loads in flight, and their sums are added in a fixed tree. The reference's
+// sqrt, its two divisions by h^2 and its division by rho_j are gone from the pair: r^2 is not rooted
+// and squared again, 1 / h^2 and the Gaussian's factor are the particle's, m / rho_j is in the record.
+// Pair stage with it at 23,416 particles: 60.4 us before (this kernel 39.8, one thread per particle),
+// 33.8 so.
 template <int BS, int G>
 __device__ __forceinline__ void pse_body(const params &P, const dev_buffers &D, blk bk) {
-  constexpr int U = G == 4 ? 2 : 4, GROUPS = BS / G;
+  constexpr int U = G == 4 ? 2 : 4;
   const int sub = (int)threadIdx.x & (G - 1);
   const double *__restrict__ rec = D.rec;
   const int N = P.N;
   const geom g = *D.g;
   const long long tex_elems = ((long long)sizeof(int) * P.N) / 8;
-  for (int q0 = bk.x * GROUPS; q0 < N; q0 += bk.n * GROUPS) {
-    const int q = q0 + (int)threadIdx.x / G, qc = min(q, N - 1);
-    const double2 fx = rec_plane(rec, 7, qc), xy = rec_plane(rec, 0, qc);
-    const double hi = rec_plane(rec, 5, qc).x;
-    const int hashi = D.hash_cur[qc];
-    const unsigned fi = (unsigned)__double_as_longlong(fx.y);
-    const bool act = q < N && !(fi & FLAG_BLANKED);
-    const double h2 = hi * hi, neg_inv_h2 = -1. / h2;
-    const int gi = hashi / g.ny;
-    const int gj = hashi - gi * g.ny;
-    const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
-    double sum = 0.;
-    if (act) {
-      for (int ii = max(gi - 2, 0); ii < min(gi + 3, g.nx); ++ii) {
-        const int j0 = __ldg(D.off + ii * g.ny + low_j);
-        const int j1 = __ldg(D.off + ii * g.ny + high_j);
-        for (int jb = j0 + sub; jb < j1; jb += U * G) {
-          double2 p[U], tf[U], cv[U];
+  const int q = bk.x * (BS / G) + (int)threadIdx.x / G, qc = min(q, N - 1);
+  const double2 fx = rec_plane(rec, 7, qc), xy = rec_plane(rec, 0, qc);
+  const double hi = rec_plane(rec, 5, qc).x;
+  const int hashi = D.hash_cur[qc];
+  const unsigned fi = (unsigned)__double_as_longlong(fx.y);
+  const bool act = q < N && !(fi & FLAG_BLANKED);
+  const double h2 = hi * hi, neg_inv_h2 = -1. / h2;
+  const int gi = hashi / g.ny;
+  const int gj = hashi - gi * g.ny;
+  const int low_j = max(gj - 2, 0), high_j = min(gj + 3, g.ny);
+  double sum = 0.;
+  if (act) {
+    for (int ii = max(gi - 2, 0); ii < min(gi + 3, g.nx); ++ii) {
+      const int j0 = __ldg(D.off + ii * g.ny + low_j);
+      const int j1 = __ldg(D.off + ii * g.ny + high_j);
+      for (int jb = j0 + sub; jb < j1; jb += U * G) {
+        double2 p[U], tf[U], cv[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int j = jb + u * G < j1 ? jb + u * G : qc;
-            p[u] = rec_plane(rec, 0, j);
-            tf[u] = rec_plane(rec, 7, j);
-            cv[u] = rec_plane(rec, 6, j);
-          }
+        for (int u = 0; u < U; ++u) {
+          const int j = jb + u * G < j1 ? jb + u * G : qc;
+          p[u] = rec_plane(rec, 0, j);
+          tf[u] = rec_plane(rec, 7, j);
+          cv[u] = rec_plane(rec, 6, j);
+        }
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (jb + u * G >= j1) continue;
-            const double dx = xy.x - p[u].x, dy = xy.y - p[u].y;
-            const double w = exp(__dmul_rn(fma(dx, dx, __dmul_rn(dy, dy)), neg_inv_h2));
-            sum = fma(__dmul_rn(__dsub_rn(tf[u].x, fx.x), cv[u].y), w, sum);
-          }
+        for (int u = 0; u < U; ++u) {
+          if (jb + u * G >= j1) continue;
+          const double dx = xy.x - p[u].x, dy = xy.y - p[u].y;
+          const double w = exp(__dmul_rn(fma(dx, dx, __dmul_rn(dy, dy)), neg_inv_h2));
+          sum = fma(__dmul_rn(__dsub_rn(tf[u].x, fx.x), cv[u].y), w, sum);
         }
       }
     }
+  }
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (act && sub == 0) {
-      const bool tool_i = q < tex_elems ? (fi & FLAG_TOOL) != 0 : false;
-      const double alpha = tool_i ? P.trml_tool.alpha : P.trml_wp.alpha;
-      const double norm = 4. / (__dmul_rn(h2, h2) * 3.14159265358979323846);
-      D.B.T_t[q] = __dmul_rn(alpha, __dmul_rn(norm, sum));
-    }
+  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (act && sub == 0) {
+    const bool tool_i = q < tex_elems ? (fi & FLAG_TOOL) != 0 : false;
+    const double alpha = tool_i ? P.trml_tool.alpha : P.trml_wp.alpha;
+    const double norm = 4. / (__dmul_rn(h2, h2) * 3.14159265358979323846);
+    D.B.T_t[q] = __dmul_rn(alpha, __dmul_rn(norm, sum));
   }
 }
 

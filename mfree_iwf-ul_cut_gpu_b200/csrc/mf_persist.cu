@@ -119,27 +119,27 @@ __global__ void __launch_bounds__(PERSIST_BLOCK, 2) kp_batch_mixed(persist_args 
   close_shared &s_close = *reinterpret_cast<close_shared *>(s_list);
   for (int st = 0; st < A.K; ++st) {
     const batch_entry *ent = A.e + (size_t)(st & 1) * A.n;
-    const batch_map m_scan{ent, A.first, A.n}, m_256{ent, A.first + (A.n + 1), A.n},
-        m_pair{ent, A.first + 2 * (A.n + 1), A.n}, m_pl{ent, A.first + 3 * (A.n + 1), A.n};
-    persist_phase(m_scan, A.grid[0], s, [&](blk b) { scan_body(s.D, s.P.N, 0, b); });
+    auto map = [&](int m) { return batch_map{ent, A.first + m * (A.n + 1), A.n}; };
+    const batch_map m_scan = map(MAP_SCAN), m_256 = map(MAP_256), m_pair = map(MAP_PAIR), m_pl = map(MAP_PLASTIC);
+    persist_phase(m_scan, A.grid[MAP_SCAN], s, [&](blk b) { scan_body(s.D, s.P.N, 0, b); });
     if (!persist_sync(A)) return;
-    persist_phase(m_256, A.grid[1], s, [&](blk b) { scatter_body(s.P.N, s.D, 0, b); });
+    persist_phase(m_256, A.grid[MAP_256], s, [&](blk b) { scatter_body(s.P.N, s.D, 0, b); });
     if (!persist_sync(A)) return;
-    persist_phase(m_256, A.grid[1], s, [&](blk b) { reorder_body<true, true>(s.P, s.D, b); });
+    persist_phase(m_256, A.grid[MAP_256], s, [&](blk b) { reorder_body<true, true>(s.P, s.D, b); });
     if (!persist_sync(A)) return;
-    persist_phase(m_pair, A.grid[2], s, [&](blk b) { pair_mixed_system<PERSIST_BLOCK>(s.P, s.D, b, s_list); });
+    persist_phase(m_pair, A.grid[MAP_PAIR], s, [&](blk b) { pair_mixed_system<PERSIST_BLOCK>(s.P, s.D, b, s_list); });
     if (!persist_sync(A)) return;
     if (A.pse) {
-      persist_phase(m_pair, A.grid[2], s, [&](blk b) { pse_mixed_system<PERSIST_BLOCK>(s.P, s.D, b); });
+      persist_phase(map(MAP_PSE), A.grid[MAP_PSE], s, [&](blk b) { pse_mixed_system<PERSIST_BLOCK>(s.P, s.D, b); });
       if (!persist_sync(A)) return;
     }
-    persist_phase(m_256, A.grid[1], s, [&](blk b) { finish_flat_body<true, false, false, false>(s.P, s.D, b, nullptr); });
+    persist_phase(m_256, A.grid[MAP_256], s, [&](blk b) { finish_flat_body<true, false, false, false>(s.P, s.D, b, nullptr); });
     if (!persist_sync(A)) return;
     if (A.plastic) {
-      if (A.paired) persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<true>(s.P, s.D, b, s_close); });
-      else persist_phase(m_pl, A.grid[3], s, [&](blk b) { plastic_body<false>(s.P, s.D, b, s_close); });
+      if (A.paired) persist_phase(m_pl, A.grid[MAP_PLASTIC], s, [&](blk b) { plastic_body<true>(s.P, s.D, b, s_close); });
+      else persist_phase(m_pl, A.grid[MAP_PLASTIC], s, [&](blk b) { plastic_body<false>(s.P, s.D, b, s_close); });
     } else {
-      persist_phase(m_pl, A.grid[3], s, [&](blk b) { close_step(s.P, s.D, finish_blocks(s.P.N), s_close); });
+      persist_phase(m_pl, A.grid[MAP_PLASTIC], s, [&](blk b) { close_step(s.P, s.D, finish_blocks(s.P.N), s_close); });
     }
     if (st + 1 < A.K && !persist_sync(A)) return;
   }

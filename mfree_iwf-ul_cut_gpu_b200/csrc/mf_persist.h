@@ -13,9 +13,9 @@ static_assert(PERSIST_BLOCK == SCAN_THREADS && PERSIST_BLOCK == BLOCK && PERSIST
 
 struct persist_args {
   const batch_entry *e;  // [2][n] entries, by buffer parity
-  const int *first;      // 4 block maps of n + 1 entries: scan, 256-thread phases, pair, plastic
+  const int *first;      // NUM_MAPS block maps of n + 1 entries
   int n, K;              // systems, steps per launch
-  int grid[4];           // blocks of each map's phase over all systems
+  int grid[NUM_MAPS];    // blocks of each map's phase over all systems
   int pse, plastic, paired;
   unsigned long long *bar;     // barrier word: arrivals, abort bit, generation
   unsigned long long wait_ns;  // limit of one barrier wait
