@@ -265,8 +265,7 @@ void set_list_mode(mf_ctx *ctx) {
 // the pair and finish kernels, where that costs most, start in turn and are spread evenly. Steps in
 // us, all early / all in turn / these two in turn: 23,416 particles FP64 45.8 / 43.2 / 42.7; 31,261
 // mixed on lists 41.9 / 38.4 / 37.1; 45,052 mixed sorted 49.6 / 45.5 / 45.2; 176,695 FP64 128.0 /
-// 125.5 / 124.3; 7,096 and 6,149 equal. (A batch's kernels, many waves each, all start early: 198.4
-// against 199.7 us a step for 24 systems.)
+// 125.5 / 124.3; 7,096 and 6,149 equal. (A batch decides by its grids: batch_start.)
 enum start { IN_TURN = 0, EARLY = 1 };
 
 // the attribute of a launch that may start early; its count for cfg.numAttrs
@@ -1137,26 +1136,43 @@ bool batch_can_fuse(mf_batch *b) {
 
 extern "C++" {  // (this part of the file lies inside the C ABI's extern "C" block)
 template <typename... KArgs, typename... Args>
-int batch_kernel(mf_batch *b, void (*kernel)(KArgs...), int grid, int block, Args... args) {
+int batch_kernel(mf_batch *b, start when, void (*kernel)(KArgs...), int grid, int block, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
   cfg.stream = b->stream;
   cudaLaunchAttribute attr;
-  cfg.numAttrs = (unsigned)start_attribute(EARLY, attr);
+  cfg.numAttrs = (unsigned)start_attribute(when, attr);
   cfg.attrs = &attr;
   return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? MF_OK : MF_ERR_CUDA;
+}
+
+// How a batch's pair and finish kernels start: in turn while their grid is one wave at most, where
+// an early start packs it on some of the SMs (as in a single system's step), early beyond. Per step
+// in mixed precision, early / in turn: 32 systems of 1.2k particles 61.0 / 53.8 us (without yielding
+// material 57.8 / 51.0; one thread per particle, before the lanes, 55.3), 8 of 6k 61.0 / 52.9, 2 of 45k
+// (95 % of a wave) 59.7 / 58.3; 3 of 38k (1.2 waves) 76.6 / 75.3, with the PSE solver 83.4 / 87.0; 2 of
+// 177k 166.9 / 167.7.
+template <typename... KArgs>
+start batch_start(const mf_batch *b, void (*kernel)(KArgs...), int grid, int block) {
+  int resident = 0;
+  const bool known = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, block, 0) == cudaSuccess;
+  return known && grid <= resident * b->ctx[0]->sm_count ? IN_TURN : EARLY;
+}
+template <typename... KArgs, typename... Args>
+int batch_wave(mf_batch *b, void (*kernel)(KArgs...), int grid, int block, Args... args) {
+  return batch_kernel(b, batch_start(b, kernel, grid, block), kernel, grid, block, args...);
 }
 
 // the pair phase (and PSE) of one step at the tuned block size
 template <int BS>
 int batch_pair(mf_batch *b, const params &P0, batch_map m, batch_map m_pse) {
   const bool mixed = P0.precision == MF_PRECISION_MIXED;
-  if (mixed) TRY(batch_kernel(b, kb_pair_mixed<BS>, b->grid[MAP_PAIR], BS, m));
-  else TRY(batch_kernel(b, kb_pair_fp64<BS>, b->grid[MAP_PAIR], BS, m));
+  if (mixed) TRY(batch_wave(b, kb_pair_mixed<BS>, b->grid[MAP_PAIR], BS, m));
+  else TRY(batch_wave(b, kb_pair_fp64<BS>, b->grid[MAP_PAIR], BS, m));
   if (P0.thermal_solver == MF_THERMAL_PSE && P0.thermal_wp) {
-    if (mixed) TRY(batch_kernel(b, kb_pse_mixed<BS>, b->grid[MAP_PSE], BS, m_pse));
-    else TRY(batch_kernel(b, kb_pse<BS>, b->grid[MAP_PSE], BS, m_pse));
+    if (mixed) TRY(batch_kernel(b, EARLY, kb_pse_mixed<BS>, b->grid[MAP_PSE], BS, m_pse));
+    else TRY(batch_kernel(b, EARLY, kb_pse<BS>, b->grid[MAP_PSE], BS, m_pse));
   }
   return MF_OK;
 }
@@ -1248,10 +1264,10 @@ int batch_build_fused(mf_batch *b, int K) {
     const batch_entry *ent = b->d_entries + (size_t)(st & 1) * n;
     auto map = [&](int m) { return batch_map{ent, b->d_first + m * (n + 1), n}; };
     const batch_map m_scan = map(MAP_SCAN), m_256 = map(MAP_256), m_pl = map(MAP_PLASTIC);
-    rc = batch_kernel(b, kb_scan, b->grid[MAP_SCAN], SCAN_THREADS, m_scan);
-    if (rc == MF_OK) rc = batch_kernel(b, kb_scatter, b->grid[MAP_256], BLOCK, m_256);
-    if (rc == MF_OK) rc = mixed ? batch_kernel(b, kb_reorder<true>, b->grid[MAP_256], BLOCK, m_256)
-                                : batch_kernel(b, kb_reorder<false>, b->grid[MAP_256], BLOCK, m_256);
+    rc = batch_kernel(b, EARLY, kb_scan, b->grid[MAP_SCAN], SCAN_THREADS, m_scan);
+    if (rc == MF_OK) rc = batch_kernel(b, EARLY, kb_scatter, b->grid[MAP_256], BLOCK, m_256);
+    if (rc == MF_OK) rc = mixed ? batch_kernel(b, EARLY, kb_reorder<true>, b->grid[MAP_256], BLOCK, m_256)
+                                : batch_kernel(b, EARLY, kb_reorder<false>, b->grid[MAP_256], BLOCK, m_256);
     if (rc == MF_OK) {
       switch (b->pair_bs) {
         case 64: rc = batch_pair<64>(b, P0, map(MAP_PAIR), map(MAP_PSE)); break;
@@ -1259,12 +1275,12 @@ int batch_build_fused(mf_batch *b, int K) {
         default: rc = batch_pair<128>(b, P0, map(MAP_PAIR), map(MAP_PSE)); break;
       }
     }
-    if (rc == MF_OK) rc = batch_kernel(b, kb_finish, b->grid[MAP_256], FINISH_BLOCK, m_256);
+    if (rc == MF_OK) rc = batch_wave(b, kb_finish, b->grid[MAP_256], FINISH_BLOCK, m_256);
     if (rc == MF_OK && P0.plastic)
-      rc = P0.jc_model == MF_JC_TANH ? batch_kernel(b, kb_plastic<false>, b->grid[MAP_PLASTIC], BLOCK, m_pl)
-                                     : batch_kernel(b, kb_plastic<true>, b->grid[MAP_PLASTIC], BLOCK, m_pl);
+      rc = P0.jc_model == MF_JC_TANH ? batch_kernel(b, EARLY, kb_plastic<false>, b->grid[MAP_PLASTIC], BLOCK, m_pl)
+                                     : batch_kernel(b, EARLY, kb_plastic<true>, b->grid[MAP_PLASTIC], BLOCK, m_pl);
     else if (rc == MF_OK)
-      rc = batch_kernel(b, kb_close, b->grid[MAP_PLASTIC], BLOCK, m_pl);
+      rc = batch_kernel(b, EARLY, kb_close, b->grid[MAP_PLASTIC], BLOCK, m_pl);
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
