@@ -527,10 +527,15 @@ __device__ __forceinline__ void predict_particle(const params &P, const dev_buff
 
   if (MIXED) {
     // FP32 record: position relative to the origin of the particle's own cell, temperature
-    // relative to the initial temperature (only differences of T enter the pair sums)
+    // relative to the initial temperature (only differences of T enter the pair sums). The origins
+    // lie dx rounded to float apart, the step with which the pair sums count columns and rows: with
+    // dx itself every pair across a cell bound was longer by dx's rounding (up to 6e-8 dx), an error
+    // of one sign that a uniform stress does not cancel. (Velocities and stresses of 210 cuts of 2k
+    // to 38k particles after 32 steps: rms error against 64 bits 0.75 and 0.78 of what it was.)
     const geom g = *D.g;
     const int ci = hsh / g.ny, cj = hsh - ci * g.ny;
-    const double ox = g.bbmin_x + ci * g.dx, oy = g.bbmin_y + cj * g.dx;
+    const double dxf = (double)(float)g.dx;
+    const double ox = g.bbmin_x + ci * dxf, oy = g.bbmin_y + cj * dxf;
     fr[F_X] = (float)(pos.x - ox);
     fr[F_Y] = (float)(pos.y - oy);
     fr[F_ROW] = blanked ? __int_as_float(0x7fffffff) : tool ? -(float)(cj + 1) : (float)(cj + 1);

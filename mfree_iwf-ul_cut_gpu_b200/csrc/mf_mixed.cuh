@@ -207,7 +207,8 @@ static __global__ void k_list_abs(int N, dev_buffers D, double2 *abs) {
   const geom g = *D.g;
   const int hj = D.hash_cur[j];
   const int cx = hj / g.ny, cy = hj - cx * g.ny;
-  abs[j] = make_double2(g.bbmin_x + cx * g.dx + (double)b0.x, g.bbmin_y + cy * g.dx + (double)b0.y);
+  const double dxf = (double)(float)g.dx;
+  abs[j] = make_double2(g.bbmin_x + cx * dxf + (double)b0.x, g.bbmin_y + cy * dxf + (double)b0.y);
 }
 
 static __global__ void k_list_check(params P, dev_buffers D, const double2 *__restrict__ abs,
