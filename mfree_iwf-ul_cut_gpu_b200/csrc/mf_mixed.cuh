@@ -593,14 +593,18 @@ __device__ __forceinline__ void pair_mixed_body(const params &P, const dev_buffe
 }
 
 // Parts of a particle's sums, and lanes per particle of the single-system kernels: as many as let
-// every particle's lanes be resident at once (24 warps per SM on 148 SMs: 28,416 particles at 4;
-// 20 warps of the list form: 47,360 at 2), then one; see pair64_lanes. Pair stage in us (launch
-// included) sorted every step / on lists, at 1 lane: 7,096 particles 19.5 / 21.5; 23,416 23.5 / 22.1;
-// 45,052 27.6 / 24.2; 70,316 31.7 / 27.7; 176,695 55 / 49; at 2: 17.4 / 17.3; 19.5 / 17.4; 23.6 /
-// 21.4; 31.7 / 31.6; 58 / 60; at 4: 15.4 / 13.3; 17.4 / 14.3; 25.6 / 21.5; 35.8 / 29.7; 71 / 67.
-// (Before, one thread per particle: 22.0 on lists at 6,149, 32.8 sorted at 45,052, 52 on lists at 176,695.)
-// A batch of many small systems fills the GPU anyway and runs them at one lane, in as many parts
-// (24 systems of 2.8k to 38k particles: 196 us a step at one lane, 209 at two, 253 at four).
+// every particle's lanes be resident at once, then one; see pair64_lanes. The sorted and the list form
+// give the same bits, so one rule serves both: the four-lane limit is the window form's (24 warps per
+// SM on 148 SMs: 28,416 particles; the list form's own, at 20 warps, is 23,680), the two-lane limit the
+// list form's (47,360; the window form's own is 56,832). Between them the other form gives away up to
+// 6 %. Step in us, sorted every step, at 4 / 2 / 1 lanes: 7,090 particles 32.9 / 34.9 / 39.0; 23,437
+// 35.4 / 37.6 / 41.3; 27,963 37.0 / 37.2 / 41.1; 28,957 39.3 / 39.0 / 41.3; 35,947 43.1 / 40.5 / 43.0;
+// 47,207 46.2 / 43.2 / 45.3; 47,978 46.5 / 43.3 / 45.2; 56,867 49.3 / 46.4 / 49.4; 64,105 52.3 / 49.3 /
+// 47.7; on lists: 28.8 / 31.4 / 36.6; 30.9 / 33.9 / 38.8; 35.9 / 34.0 / 39.1; 37.0 / 35.4 / 39.5; 37.4 /
+// 35.4 / 40.5; 39.5 / 37.8 / 43.0; 43.2 / 43.9 / 43.6; 46.1 / 48.0 / 43.6; 47.0 / 49.3 / 44.5.
+// (Before, one thread per particle: pair stage 22.0 on lists at 6,149, 32.8 sorted at 45,052.)
+// A batch of many small systems fills the GPU anyway and runs the pair sums at one lane, in as many
+// parts (24 systems of 2.8k to 38k particles: 196 us a step at one lane, 209 at two, 253 at four).
 __host__ __device__ constexpr int mixed_parts(int N) { return N <= 28416 ? 4 : N <= 47360 ? 2 : 1; }
 
 // blocks per SM: the window form at 6 (80 registers, no spills), the list form at 5 (96 registers,
@@ -621,7 +625,7 @@ static __global__ void __launch_bounds__(PAIR_BLOCK, LIST ? 5 : 6) k_pair_mixed(
 // It is bound by instructions (56 candidates of a particle), so a round of 8 candidates is read at
 // constant offsets from one address (past the column's end what is read is not used), and a blanked
 // candidate, whose record holds no row, is noticed by the NaN it leaves and the round done again.
-// Measured at 577,555 particles: 54.9 us before (41 instructions a candidate), 48.3 so.
+// Measured at 577,555 particles: 54.9 us before (41 instructions a candidate), 46.4 so.
 template <int BS, int G>
 __device__ __forceinline__ void pse_mixed_body(const params &P, const dev_buffers &D, blk bk) {
   constexpr int U = 8 / G;

@@ -774,8 +774,13 @@ cudaError_t launch(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, int
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// lanes per particle of the pair kernel, by the particle count alone, so that a pass with one
-// direction and one with six add each direction up alike
+// Lanes per particle of the pair kernel, by the particle count alone, so that a pass with one
+// direction and one with six add each direction up alike. As many as let one direction's lanes be
+// resident at once (4 blocks of 64 per SM: 9,472 particles at 4, 18,944 at 2), the four-lane limit
+// lower, because six directions fill the GPU anyway and lose by four lanes at every size. Step in us
+// at 4 / 2 / 1 lanes, one direction: 3,467 particles 68 / 75 / 95; 8,329 68 / 79 / 99; 11,233 86 / 81 /
+// 101; 18,822 92 / 85 / 108; 23,437 108 / 104 / 107; 31,203 124 / 115 / 112; six: 97 / 91 / 103; 152 /
+// 137 / 145; 196 / 170 / 162; 303 / 252 / 229; 368 / 304 / 278; 483 / 396 / 355.
 constexpr int lanes(int N) { return N <= 8192 ? 4 : N <= 18944 ? 2 : 1; }
 
 // Work memory kept for a context's next call; a larger one is given back, so that contexts with many
